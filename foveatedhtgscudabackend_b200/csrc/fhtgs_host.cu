@@ -146,7 +146,7 @@ struct Layout {
     size_t off_hist, off_dtot, off_ranges, off_map, off_type, off_ltype, off_wf, off_wl, off_wm, off_ctr, off_temp;
     size_t off_order0, off_order1;
     size_t off_ghist, off_look, off_ticket;
-    size_t off_split_of = 0, off_split_list = 0, off_split_ctl = 0, off_split_scratch = 0, off_split_status = 0;
+    size_t off_split_of = 0, off_split_list = 0, off_split_ctl = 0, off_split_scratch = 0;
     size_t off_split_units = 0, off_split_pool = 0;
     std::vector<size_t> temp_offsets;
 };
@@ -167,7 +167,7 @@ SplitPlan split_plan(float share, int recs, int exact, int64_t pool, int K, int 
     sp.exact = exact;
     if (exact) sp.pool_units = static_cast<uint32_t>((pool > 0 ? pool : kSplitPoolDefault) / 256);
     const int Ki = K >= 32 ? 32 : K >= 16 ? 16 : K >= 8 ? 8 : K >= 4 ? 4 : K >= 2 ? 2 : 1;  // the blend's K
-    const int per_sm = blend_blocks_per_sm > 0 ? std::min(blend_blocks_per_sm, blend_min_blocks(Ki)) : blend_min_blocks(Ki);
+    const int per_sm = blend_blocks_per_sm > 0 ? std::min(blend_blocks_per_sm, split_share_blocks(Ki)) : split_share_blocks(Ki);
     sp.share = share;
     sp.blocks = n_sms * per_sm;
     sp.recs = exact ? 0 : recs > 0 ? recs : 8 * Ki + 64;  // 20 bytes each
@@ -205,8 +205,8 @@ Layout plan(int V, int64_t N, int nbp, int64_t cap, int key_bytes, int sort_tile
     L.off_wl = take(4ull * V * max_large);
     L.off_wm = take(4ull * V * max_large);
     L.off_ctr = take(4ull * kCounterWords);
-    L.off_order0 = take(4ull * V * max_large);
-    L.off_order1 = take(4);
+    L.off_order0 = take(8ull * V * max_large);
+    L.off_order1 = take(4ull * V * max_large);
     L.off_ghist = take(4ull * V * kSortMaxPasses * kSortBins);
     L.off_look = take(4ull * V * kSortMaxPasses * sort_tiles * kSortBins);
     L.off_ticket = take(4ull * V * kSortMaxPasses);
@@ -216,7 +216,6 @@ Layout plan(int V, int64_t N, int nbp, int64_t cap, int key_bytes, int sort_tile
         L.off_split_list = take(8ull * sp.cap);
         L.off_split_ctl = take(4ull * sp.cap);
         L.off_split_scratch = take(static_cast<size_t>(sp.stride) * sp.cap);
-        L.off_split_status = take(sizeof(FrameStatus) * V);
         L.off_split_units = take(4ull * sp.cap);
         L.off_split_pool = take(256ull * sp.pool_units);
     }
@@ -432,7 +431,6 @@ fhtgs_status render_impl(fhtgs_context ctx, const fhtgs_primitives* prims, const
         sa.list = reinterpret_cast<uint2*>(A + L.off_split_list);
         sa.ctl = reinterpret_cast<uint32_t*>(A + L.off_split_ctl);
         sa.scratch = A + L.off_split_scratch;
-        sa.status = reinterpret_cast<FrameStatus*>(A + L.off_split_status);
         sa.exact = P.split.exact;
         sa.pool_units = P.split.pool_units;
         sa.seg_unit = reinterpret_cast<uint32_t*>(A + L.off_split_units);

@@ -13,8 +13,8 @@
 // The reference stores the four sub-tiles of every fovea tile as separate instances with
 // identical lists, plus sentinel slots for masked fovea tiles; here each list is stored once
 // and the reference's arrays are reproduced exactly on request (fhtgs_copy_intermediates).
-//   blend      K-buffer blend; full-res 16x16 tiles (fovea, blended) and 2x-down 16x16
-//              tiles (periphery), persistent blocks pulling tiles from a work counter
+//   blend      K-buffer blend; full-res 16x16 tiles (fovea, blended) and strided 16x16 tiles
+//              (periphery, quarter), persistent blocks pulling items from a work counter
 //   compose    periphery bilinear upsampling / blur and blended-ring cross-fade
 #pragma once
 #include <cuda_bf16.h>
@@ -1309,20 +1309,51 @@ int launch_ranges(const FrameParams& fp, const FrameBuffers& fb, int n_sms, cuda
 
 // ------------------------------------------------------------------------------------------
 // work ordering for the persistent blend (bucketed longest-processing-time first)
-// One list holds both kinds of tile: full-resolution (fovea + blended, 8 warps of pixels) and
-// periphery (8 x 8 samples at stride 2, 2 warps).  An item is packed as
-//   view << 24 | periphery << 23 | index into the view's work_full / work_low list.
-// Its cost is (warps x list length); items are bucketed by cost in quarter octaves and the
-// buckets are served heaviest first, so that long serial per-pixel chains start early.
+// One list of block items, longest estimated duration first, so that the serial walks of the
+// long lists start early and the short ones fill the end:
+//   full    a full-resolution tile, two pixels a thread
+//   half    the upper or lower half of a full-resolution tile, one pixel a thread: the tiles
+//           whose walk alone would outlast the frame's mean work per block
+//   low     four periphery tiles, one per warp
+//   quarter sixteen ring-mode quarter tiles, four per warp
+// An item word is kind << 29 | view << 21 | index into the view's work_full list, or kind << 29 |
+// item number for the last two, whose tiles lie in work_order[1] (view << 21 | index into
+// work_low), longest first: the periphery tiles of all views, then the quarter tiles.
 // ------------------------------------------------------------------------------------------
-constexpr uint32_t kItemLowres = 1u << 23;
+constexpr uint32_t kItemFull = 0u, kItemHalf = 1u /* and 2 */, kItemLow = 3u, kItemQuarter = 4u;
+constexpr int kItemKindShift = 29, kItemViewShift = 21;
+constexpr uint32_t kItemIndexMask = (1u << kItemViewShift) - 1u;
+constexpr uint32_t kItemNumberMask = (1u << kItemKindShift) - 1u;
+__device__ __forceinline__ int item_view(uint32_t packed) { return static_cast<int>((packed >> kItemViewShift) & 255u); }
+__device__ __forceinline__ uint32_t item_index(uint32_t packed) { return packed & kItemIndexMask; }
+// Tiles of a low / quarter item.
+constexpr uint32_t kLowTiles = 4, kQuarterTiles = 16;
+
+// Estimated duration of an item in list entries of a full item: per entry of its (longest) list,
+// plus the item's fixed cost.  Measured on the stereo frames: 148 ns per entry of a full item and
+// 115 of a half item at four blocks per SM, 230 of a periphery item, about 5 us fixed.
+constexpr float kCostHalf = 0.75f, kCostLow = 1.6f, kCostQuarter = 2.5f, kCostItem = 32.0f;
+// A full-resolution tile becomes two half items when its list is longer than this share of the
+// frame's instances per SM: its walk would then outlast the frame at five blocks per SM.
+constexpr float kHalfShare = 0.16f;
+
+// Resident blocks per SM.  More blocks hide more latency (relative throughput of 1 to 5 blocks,
+// measured on a 12-view frame: 1, 1.75, 2.29, 2.64, 2.86), but each block then walks slower, and
+// a frame ends with its longest item.  With u = longest item / (all items per SM), the time at b
+// blocks is about max(1 / throughput(b), u b / throughput(b)): the limits below are where b blocks
+// become better than b + 1.  (Plain view, u = 1.2: blend 0.34 -> 0.20 ms at one block; half-size
+// stereo frame, u = 0.38: 2.43 -> 1.84 ms at three.)
+__device__ __forceinline__ uint32_t blocks_per_sm(float u, uint32_t most) {
+    const uint32_t b = u < 0.21f ? 5u : u < 0.29f ? 4u : u < 0.43f ? 3u : u < 0.87f ? 2u : 1u;
+    return b < most ? b : most;
+}
 
 __device__ __forceinline__ int items_of_view(const FrameStatus& st) {
     return static_cast<int>(st.n_fovea_large + st.n_blended_large + st.n_periphery_large + st.n_quarter_large);
 }
 
-__device__ __forceinline__ int cost_bucket(uint32_t cost) {
-    return cost == 0 ? 0 : min(kCostBuckets - 1, 1 + __float2int_rd(4.0f * __log2f(static_cast<float>(cost))));
+__device__ __forceinline__ int cost_bucket(float cost) {
+    return cost < 1.0f ? 0 : min(kCostBuckets - 1, 1 + __float2int_rd(4.0f * __log2f(cost)));
 }
 
 // Maps flat item g to (view, index within the view); `pre` holds the exclusive prefix of the
@@ -1337,9 +1368,10 @@ __device__ __forceinline__ void item_of(int g, const int* pre, int n_views, int&
     j = g - pre[lo];
 }
 
-// Packed item and cost of the view's j-th item (full-resolution tiles first).
-__device__ __forceinline__ uint32_t item_cost(const FrameParams& fp, const FrameBuffers& fb, int v, int j,
-                                              uint32_t& packed) {
+// The view's j-th tile (full-resolution tiles, then periphery, then quarter tiles): its class (2,
+// 1, 0), its list length and its view << 21 | index word.
+__device__ __forceinline__ int item_tile(const FrameParams& fp, const FrameBuffers& fb, int v, int j, uint32_t& len,
+                                         uint32_t& packed) {
     const FrameStatus& st = fb.status[v];
     const int n_full = static_cast<int>(st.n_fovea_large + st.n_blended_large);
     const bool low = j >= n_full;
@@ -1347,23 +1379,24 @@ __device__ __forceinline__ uint32_t item_cost(const FrameParams& fp, const Frame
     const uint32_t lt = low ? fb.work_low[static_cast<size_t>(v) * fp.max_large + idx]
                             : fb.work_full[static_cast<size_t>(v) * fp.max_large + idx];
     const uint2 r = fb.ranges[static_cast<size_t>(v) * fp.max_large + lt];
-    packed = (static_cast<uint32_t>(v) << 24) | (low ? kItemLowres : 0u) | static_cast<uint32_t>(idx);
-    const uint32_t len = r.y > r.x ? r.y - r.x : 0u;
-    const bool quarter = low && static_cast<uint32_t>(idx) >= st.n_periphery_large;
-    return len * (quarter ? 1u : low ? 2u : 8u);
+    packed = (static_cast<uint32_t>(v) << kItemViewShift) | static_cast<uint32_t>(idx);
+    len = r.y > r.x ? r.y - r.x : 0u;
+    return !low ? 2 : static_cast<uint32_t>(idx) < st.n_periphery_large ? 1 : 0;
 }
 
-// Work-list bucket of an item: its class (full resolution 2, periphery 1, quarter 0) above its
-// cost bucket, so that the descending scatter lists every full-resolution tile first (all 8
-// warps of a block busy), then the periphery tiles, then the quarter tiles, each class heaviest
-// first; a strided tile then never holds a block that full-resolution work is waiting for.
-__device__ __forceinline__ int item_bucket(const FrameParams& fp, const FrameBuffers& fb, int v, int j, uint32_t& packed,
-                                           uint32_t& cost) {
-    cost = item_cost(fp, fb, v, j, packed);
-    const FrameStatus& st = fb.status[v];
-    const int n_full = static_cast<int>(st.n_fovea_large + st.n_blended_large);
-    const int cls = j < n_full ? 2 : (j - n_full) < static_cast<int>(st.n_periphery_large) ? 1 : 0;
-    return cls * kCostBuckets + cost_bucket(cost);
+// Estimated duration of a tile's item (class 2: full or half), see kCostHalf.
+__device__ __forceinline__ float item_cost(int cls, uint32_t len, bool halves) {
+    const float c = cls == 2 ? (halves ? kCostHalf : 1.0f) : cls == 1 ? kCostLow : kCostQuarter;
+    return c * static_cast<float>(len) + kCostItem;
+}
+// Its bucket: class above duration bucket.
+__device__ __forceinline__ int item_bucket(int cls, float cost) { return cls * kCostBuckets + cost_bucket(cost); }
+
+// List length above which a full-resolution tile is blended as two half items.
+__device__ __forceinline__ uint32_t half_threshold(const FrameParams& fp, const FrameBuffers& fb, int n_sms) {
+    uint64_t m = 0;
+    for (int v = 0; v < fp.n_views; ++v) m += view_count(fp, fb, v);
+    return static_cast<uint32_t>(fminf(kHalfShare * static_cast<float>(m) / static_cast<float>(n_sms), 4e9f));
 }
 
 // Split blend: the list length above which a full-resolution tile is split, share x the
@@ -1416,87 +1449,135 @@ __device__ __forceinline__ int items_prefix(const FrameParams& fp, const FrameBu
 }
 
 // Also decides which full-resolution tiles the split blend splits (they leave the work list,
-// their segments go to the split list) and clears the split tickets.
-__global__ void __launch_bounds__(256) order_hist_kernel(FrameParams fp, FrameBuffers fb, SplitArgs sp) {
+// their segments go to the split list) and clears the split tickets, and adds up the items' costs.
+__global__ void __launch_bounds__(256) order_hist_kernel(FrameParams fp, FrameBuffers fb, SplitArgs sp, int n_sms) {
     __shared__ int pre[kMaxOrderViews];
     __shared__ uint32_t hist[kOrderBuckets];
-    __shared__ uint32_t s_split_len;
+    __shared__ uint32_t s_split_len, s_half_len;
+    __shared__ float s_cost[256 / 32], s_longest[256 / 32];
+    float cost_sum = 0.0f, longest = 0.0f;
     const int total = items_prefix(fp, fb, pre);
     for (int k = threadIdx.x; k < kOrderBuckets; k += blockDim.x) hist[k] = 0;
-    if (threadIdx.x == 0) s_split_len = split_threshold(fp, fb, sp);
+    if (threadIdx.x == 0) {
+        s_split_len = split_threshold(fp, fb, sp);
+        s_half_len = half_threshold(fp, fb, n_sms);
+    }
     __syncthreads();
-    const uint32_t split_len = s_split_len;
+    const uint32_t split_len = s_split_len, half_len = s_half_len;
     if (split_len > 0)
         for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < sp.cap; k += gridDim.x * blockDim.x) sp.ctl[k] = 0u;
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
         int v, j;
         item_of(g, pre, fp.n_views, v, j);
-        uint32_t packed, cost;
-        const int b = item_bucket(fp, fb, v, j, packed, cost);
-        if (split_len > 0 && b >= 2 * kCostBuckets) {  // a full-resolution tile: cost = 8 x length
-            const uint32_t len = cost / 8u;
+        uint32_t packed, len;
+        const int cls = item_tile(fp, fb, v, j, len, packed);
+        if (split_len > 0 && cls == 2) {
             uint32_t tag = ~0u, seg0;
             if (len > split_len) {
                 const uint32_t S = min(static_cast<uint32_t>(kSplitMaxSegments), (len + split_len - 1) / split_len);
                 if (split_reserve(fb, sp, S, len, seg0)) {
                     tag = seg0 | (S << 28);
                     atomicAdd(&fb.counters[kCtrSplitTiles], 1u);
-                    atomicAdd(&fb.counters[kCtrSplitView + v], 1u);
                 }
             }
             sp.of[static_cast<size_t>(v) * fp.max_large + j] = tag;
             if (tag != ~0u) continue;
         }
-        atomicAdd(&hist[b], 1u);
+        const bool halves = cls == 2 && len > half_len;
+        const float cost = item_cost(cls, len, halves);
+        longest = fmaxf(longest, cost);
+        cost_sum += cost * (cls == 2 ? (halves ? 2.0f : 1.0f) : 1.0f / (cls == 1 ? kLowTiles : kQuarterTiles));
+        atomicAdd(&hist[item_bucket(cls, cost)], halves ? 2u : 1u);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        cost_sum += __shfl_xor_sync(0xffffffffu, cost_sum, o);
+        longest = fmaxf(longest, __shfl_xor_sync(0xffffffffu, longest, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        s_cost[threadIdx.x >> 5] = cost_sum;
+        s_longest[threadIdx.x >> 5] = longest;
     }
     __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 256 / 32; ++w) {
+            cost_sum += s_cost[w];
+            longest = fmaxf(longest, s_longest[w]);
+        }
+        atomicAdd(reinterpret_cast<float*>(&fb.counters[kCtrCost]), cost_sum);
+        atomicMax(&fb.counters[kCtrLongest], __float_as_uint(longest));  // non-negative: ordered as integers
+    }
     uint32_t* gh = fb.counters + kCtrHist;
     for (int k = threadIdx.x; k < kOrderBuckets; k += blockDim.x)
         if (hist[k]) atomicAdd(&gh[k], hist[k]);
 }
 
-// Items go to their bucket's run of the work list in rounds of blockDim.x: a block counts its
-// round's items per bucket in shared memory (each item's rank among them), reserves one
-// contiguous place per bucket with a single global atomic, and writes its items there.  (One
-// global atomic per item made the few heavily used buckets' cursors a serial bottleneck.)  The
-// order inside a bucket follows the reservations; it changes the schedule, never a pixel.
-__global__ void __launch_bounds__(256) order_scatter_kernel(FrameParams fp, FrameBuffers fb, SplitArgs sp) {
+// Tiles go to their bucket's run in rounds of blockDim.x: a block counts its round's entries per
+// bucket in shared memory (each tile's rank among them), reserves one contiguous place per bucket
+// with a single global atomic, and writes them there.  (One global atomic per tile made the few
+// heavily used buckets' cursors a serial bottleneck.)  The place of a block item in the merged
+// list is its place in its own class plus the items of the other classes in longer buckets (equal
+// buckets: full, low, quarter).  The order inside a bucket follows the reservations; it changes
+// the schedule, never a pixel.
+__global__ void __launch_bounds__(256) order_scatter_kernel(FrameParams fp, FrameBuffers fb, SplitArgs sp, int n_sms,
+                                                            int max_per_sm) {
     __shared__ int pre[kMaxOrderViews];
-    __shared__ uint32_t base[kOrderBuckets];
+    __shared__ uint32_t base[kOrderBuckets + 1];  // entries in higher buckets (of this and higher classes)
     __shared__ uint32_t s_cnt[kOrderBuckets];
     __shared__ uint32_t s_warp[33];
+    __shared__ uint32_t s_half_len;
     const int total = items_prefix(fp, fb, pre);
-    if (sp.status != nullptr && sp.share > 0.0f && blockIdx.x == 0)
-        for (int v = threadIdx.x; v < fp.n_views; v += blockDim.x) {
-            FrameStatus c = fb.status[v];
-            c.n_blended_large -= fb.counters[kCtrSplitView + v];
-            sp.status[v] = c;
-        }
     const uint32_t* gh = fb.counters + kCtrHist;
     uint32_t* cursor = fb.counters + kCtrHist + kOrderBuckets;
-    {  // each bucket's first place in descending bucket order: a block scan, two buckets a thread
+    if (threadIdx.x == 0) s_half_len = half_threshold(fp, fb, n_sms);
+    uint32_t all;
+    {  // a block scan in descending bucket order, two buckets a thread
         static_assert(kOrderBuckets <= 2 * 256, "two buckets per thread of a 256-thread block");
         const int p0 = 2 * static_cast<int>(threadIdx.x), p1 = p0 + 1;  // places in descending order
         const uint32_t c0 = p0 < kOrderBuckets ? gh[kOrderBuckets - 1 - p0] : 0u;
         const uint32_t c1 = p1 < kOrderBuckets ? gh[kOrderBuckets - 1 - p1] : 0u;
-        uint32_t all;
         const uint32_t e = block_excl_scan<uint32_t>(c0 + c1, all, s_warp);
         if (p0 < kOrderBuckets) base[kOrderBuckets - 1 - p0] = e;
         if (p1 < kOrderBuckets) base[kOrderBuckets - 1 - p1] = e + c0;
     }
+    __syncthreads();
+    const uint32_t half_len = s_half_len;
+    const uint32_t n_full = base[2 * kCostBuckets - 1];  // entries above the periphery class
+    const uint32_t n_low = base[kCostBuckets - 1] - n_full, n_quarter = all - n_full - n_low;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        fb.counters[kCtrItems] = n_full + (n_low + kLowTiles - 1) / kLowTiles + (n_quarter + kQuarterTiles - 1) / kQuarterTiles;
+        fb.counters[kCtrLow] = n_low;
+        fb.counters[kCtrQuarter] = n_quarter;
+        const float u = __uint_as_float(fb.counters[kCtrLongest]) * static_cast<float>(n_sms) /
+                        fmaxf(__uint_as_float(fb.counters[kCtrCost]), 1.0f);
+        fb.counters[kCtrBlocks] = static_cast<uint32_t>(n_sms) * blocks_per_sm(u, static_cast<uint32_t>(max_per_sm));
+    }
+    // entries of a class in duration buckets >= d (d = kCostBuckets: none)
+    auto at_least = [&](int cls, int d) {
+        const uint32_t start = cls == 2 ? 0u : cls == 1 ? n_full : n_full + n_low;
+        if (d >= kCostBuckets) return 0u;
+        const int k = cls * kCostBuckets + d;
+        return (k > 0 ? base[k - 1] : all) - start;
+    };
+    auto low_items = [&](int d) { return (at_least(1, d) + kLowTiles - 1) / kLowTiles; };
+    auto quarter_items = [&](int d) { return (at_least(0, d) + kQuarterTiles - 1) / kQuarterTiles; };
     uint32_t* out = fb.work_order[0];
+    uint32_t* runs = fb.work_order[1];
     for (int g0 = blockIdx.x * blockDim.x; g0 < total; g0 += gridDim.x * blockDim.x) {
         for (int k = threadIdx.x; k < kOrderBuckets; k += blockDim.x) s_cnt[k] = 0;
         __syncthreads();
         const int g = g0 + static_cast<int>(threadIdx.x);
-        int b = -1;
+        int b = -1, cls = 0;
+        bool halves = false;
         uint32_t packed = 0, local = 0;
         if (g < total) {
             int v, j;
             item_of(g, pre, fp.n_views, v, j);
-            uint32_t cost;
-            b = item_bucket(fp, fb, v, j, packed, cost);
-            if (sp.of != nullptr && sp.share > 0.0f && b >= 2 * kCostBuckets) {
+            uint32_t len;
+            cls = item_tile(fp, fb, v, j, len, packed);
+            halves = cls == 2 && len > half_len;
+            b = item_bucket(cls, item_cost(cls, len, halves));
+            if (sp.of != nullptr && sp.share > 0.0f && cls == 2) {
                 const uint32_t tag = sp.of[static_cast<size_t>(v) * fp.max_large + j];
                 if (tag != ~0u) {  // a split tile: its segments go to the split list
                     const uint32_t seg0 = tag & 0x0fffffffu, S = tag >> 28;
@@ -1504,47 +1585,90 @@ __global__ void __launch_bounds__(256) order_scatter_kernel(FrameParams fp, Fram
                     b = -1;
                 }
             }
-            if (b >= 0) local = atomicAdd(&s_cnt[b], 1u);
+            if (b >= 0) local = atomicAdd(&s_cnt[b], halves ? 2u : 1u);
         }
         __syncthreads();
         for (int k = threadIdx.x; k < kOrderBuckets; k += blockDim.x)
             if (s_cnt[k]) s_cnt[k] = atomicAdd(&cursor[k], s_cnt[k]);
         __syncthreads();
-        if (b >= 0) out[base[b] + s_cnt[b] + local] = packed;
+        if (b >= 0) {
+            const uint32_t at = base[b] + s_cnt[b] + local;  // place among all entries, classes one after the other
+            const int d = b - cls * kCostBuckets;
+            if (cls == 2) {
+                const uint32_t place = at + low_items(d + 1) + quarter_items(d + 1);
+                if (halves) {
+                    out[place] = (kItemHalf << kItemKindShift) | packed;
+                    out[place + 1] = ((kItemHalf + 1u) << kItemKindShift) | packed;
+                } else {
+                    out[place] = (kItemFull << kItemKindShift) | packed;
+                }
+            } else {
+                runs[at - n_full] = packed;
+                const uint32_t per = cls == 1 ? kLowTiles : kQuarterTiles, k = at - n_full - (cls == 1 ? 0u : n_low);
+                if (k % per == 0)  // the first tile of an item
+                    out[k / per + at_least(2, d) + (cls == 1 ? quarter_items(d + 1) : low_items(d))] =
+                        ((cls == 1 ? kItemLow : kItemQuarter) << kItemKindShift) | (k / per);
+            }
+        }
         __syncthreads();  // the counts are cleared for the next round
     }
 }
 
 int launch_order(const FrameParams& fp, const FrameBuffers& fb, const SplitArgs& sp, int n_sms, cudaStream_t s) {
     const int per_view = fp.max_large;
-    int blocks = (fp.n_views * per_view + 255) / 256;
-    blocks = blocks < 2 * n_sms ? (blocks > 0 ? blocks : 1) : 2 * n_sms;
-    order_hist_kernel<<<blocks, 256, 0, s>>>(fp, fb, sp);
-    order_scatter_kernel<<<blocks, 256, 0, s>>>(fp, fb, sp);
+    int grid = (fp.n_views * per_view + 255) / 256;
+    grid = grid < 2 * n_sms ? (grid > 0 ? grid : 1) : 2 * n_sms;
+    const int per_sm = blend_blocks(fp.K);
+    order_hist_kernel<<<grid, 256, 0, s>>>(fp, fb, sp, n_sms);
+    order_scatter_kernel<<<grid, 256, 0, s>>>(fp, fb, sp, n_sms,
+                                              fp.blend_blocks > 0 && fp.blend_blocks < per_sm ? fp.blend_blocks : per_sm);
     return 2;
 }
 
 // ------------------------------------------------------------------------------------------
 // K-buffer blend (restates blend_cu and FragmentInfo, inference.cuh:16-286, and the
 // background models, background_model.cuh:8-117).  Per pixel the arithmetic and the order of
-// Gaussians are the reference's; a Gaussian is skipped for a whole warp when the warp's pixel
-// rectangle lies outside the Gaussian's cutoff ellipse bounding box (+1 px), where every pixel
-// would fail the alpha >= 1/255 test anyway.
+// Gaussians are the reference's; a Gaussian is skipped for a group of 16 pixels when the group's
+// rectangle lies outside the Gaussian's cutoff ellipse, where every pixel would fail the
+// alpha >= 1/255 test anyway.
+//
+// Bound: FP32 instruction issue.  What the design takes out of it, against one pixel a lane, one
+// list per warp (8 x 4 pixels) and eight warps a tile (same images, bit for bit):
+//   - lists per 4 x 4 pixels instead of 8 x 4: 37 % instead of 43 % of the listed pairs are
+//     evaluated at 2064x2208 (19 instead of 26 % at 1280x720; 28 and 9 % pass the alpha test);
+//   - two pixels a lane in packed FP32 arithmetic: 82 instead of 2 x 70 instructions a pair of
+//     pixels, the record loads and list steps shared;
+//   - a per-Gaussian depth bound in front of the depth evaluation: a quarter of the steps
+//     evaluate it instead of half;
+//   - one x interval per row of groups instead of a test per rectangle; selections instead of
+//     branches in the K-buffer insertion;
+//   - half items and fewer blocks per SM for frames that end with a few long tiles (work order).
+// Blend of the stereo frame (1M Gaussians, 2 x 2064x2208, K = 8) 4.87 -> 3.30 ms, of 12 views of
+// 1920x1080 10.65 -> 6.65 ms, of the plain 1280x720 view (100k, K = 4) 0.73 -> 0.20 ms, of a
+// 2 x 1032x1104 frame of the 1M scene 5.3 -> 1.84 ms, K = 32 at 1280x720 0.72 -> 0.56 ms.
 // ------------------------------------------------------------------------------------------
 struct Frag {
     float depth;
     uint32_t color;
 };
 
+// A channel clamped to [0, 1] (NaN: 0) and rounded to 8 bits, in the low byte: adding 2^23 with
+// rounding down leaves the integer part in the mantissa, on the FMA pipe instead of the slower
+// conversion unit.
 __device__ __forceinline__ uint32_t pack_channel(const float x) {
-    return static_cast<uint32_t>(fminf(fmaxf(x, 0.0f), 1.0f) * 255.0f + 0.5f);
+    return __float_as_uint(__fadd_rd(__fmaf_rn(__saturatef(x), 255.0f, 0.5f), 8388608.0f));
 }
 __device__ __forceinline__ uint32_t pack_rgba(const float4 c) {
-    return pack_channel(c.x) | (pack_channel(c.y) << 8) | (pack_channel(c.z) << 16) | (pack_channel(c.w) << 24);
+    return __byte_perm(__byte_perm(pack_channel(c.x), pack_channel(c.y), 0x0040),
+                       __byte_perm(pack_channel(c.z), pack_channel(c.w), 0x0040), 0x5410);
+}
+// 2^23 + byte `i` of c as a float, less 2^23: the byte's value.
+template <int i>
+__device__ __forceinline__ float byte_value(const uint32_t c) {
+    return __uint_as_float(__byte_perm(c, 0x4B000000u, 0x7440 | i)) - 8388608.0f;
 }
 __device__ __forceinline__ float4 unpack_rgba(const uint32_t c) {
-    return make_float4(static_cast<float>((c >> 0) & 0xff), static_cast<float>((c >> 8) & 0xff),
-                       static_cast<float>((c >> 16) & 0xff), static_cast<float>((c >> 24) & 0xff)) * (1.0f / 255.0f);
+    return make_float4(byte_value<0>(c), byte_value<1>(c), byte_value<2>(c), byte_value<3>(c)) * (1.0f / 255.0f);
 }
 
 __device__ __forceinline__ float3 background_dir(const ViewParams& vp, float px, float py) {
@@ -1678,34 +1802,129 @@ __device__ __forceinline__ bool cutoff_conic(const float4 P1, const float4 P2, c
            isfinite(q.D) && isfinite(q.E) && isfinite(q.x0) && isfinite(q.y0);
 }
 
-// Does the ellipse F <= 0 meet the pixel rectangle [ax0, ax1] x [ay0, ay1]?  Minimum of the
-// convex F over the rectangle: the free minimum if it lies inside, else the best edge point.
-__device__ __forceinline__ bool conic_meets_rect(const Conic& q, float ax0, float ax1, float ay0, float ay1) {
-    const float X0 = ax0 - q.x0 - kCullPixelMargin, X1 = ax1 - q.x0 + kCullPixelMargin,
-                Y0 = ay0 - q.y0 - kCullPixelMargin, Y1 = ay1 - q.y0 + kCullPixelMargin;
-    const float xc = (q.B * q.E - 2.0f * q.C * q.D) / q.det, yc = (q.B * q.D - 2.0f * q.A * q.E) / q.det;
-    if (xc >= X0 && xc <= X1 && yc >= Y0 && yc <= Y1) return true;
-    auto F = [&](float x, float y) { return (q.A * x + q.B * y + q.D) * x + (q.C * y + q.E) * y + q.F0; };
-    const float i2a = 0.5f / q.A, i2c = 0.5f / q.C;
-    const float yl = fminf(fmaxf(-(q.B * X0 + q.E) * i2c, Y0), Y1);
-    const float yr = fminf(fmaxf(-(q.B * X1 + q.E) * i2c, Y0), Y1);
-    const float xt = fminf(fmaxf(-(q.B * Y0 + q.D) * i2a, X0), X1);
-    const float xb = fminf(fmaxf(-(q.B * Y1 + q.D) * i2a, X0), X1);
-    const float m = fminf(fminf(F(X0, yl), F(X1, yr)), fminf(F(xt, Y0), F(xb, Y1)));
-    return !(m > 0.0f);
+// How a tile's samples map onto threads.  A warp walks groups of 16 samples, each along its own
+// list of the Gaussians that may reach the group's rectangle: four groups, one per 8 lanes with
+// two samples a lane (PX 2), or two groups, one per 16 lanes (PX 1, half items).  CLS 0: a
+// full-resolution tile (16 x 16 samples, 16 groups: the whole block, or half of them for a half
+// item); CLS 1: a periphery tile (8 x 8 samples at stride 2, four groups, one warp); CLS 2: a
+// ring-mode quarter tile (4 x 4 samples at stride 4, one group: a warp blends four tiles).
+// RW (fhtgs_tuning.blend_warp_width) gives the group rectangle: 8: 4 x 4, 16: 8 x 2, 4: 2 x 8.
+template <int RW, int CLS>
+struct GroupShape {
+    static constexpr int S = CLS == 0 ? 1 : CLS == 1 ? kStride : kQuarterStride;
+    static constexpr int SIDE = kTileLarge / S;  // samples per tile row
+    static constexpr int GW = CLS == 2 ? 4 : RW == 16 ? 8 : RW == 4 ? 2 : 4, GH = 16 / GW;
+    static constexpr int COLS = SIDE / GW, ROWS = SIDE / GH;
+};
+
+__device__ __forceinline__ float rcp_approx(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float sqrt_approx(float x) {
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
 }
 
-// Shared memory of a blend block: one batch of 256 staged Gaussian records (the three VPMT rows
-// and rgba), each Gaussian's warp-culling mask, and each warp's compacted list of batch positions.
+// Which sample groups of the tile at pixel (ox, oy) the Gaussian may reach: bit row * COLS + col,
+// among `valid`.  The cutoff ellipse about its centre is x = slope y +- hx sqrt(1 - (y / ymax)^2);
+// its x extent over a row of groups gives that row's bits at once (one test per row of groups
+// instead of one per group).  Ellipses that are not clearly ellipses, or out of the range of the
+// approximate arithmetic, are tested by their bounding box; unbounded ones reach every group, and
+// so do Gaussians so small (F0 = -rc |d|^2 at the mean) that the blend's 1 / |d|^2 may overflow:
+// 0 x inf makes their alpha 1 at any pixel of their tiles.
+// Rows row0 .. row0 + ROWS_USED - 1 of groups are tested (a half item's).
+// `zmin` receives a depth that no fragment of the core (alpha >= 1/20) undercuts: the depth is
+// w4 + n4 . e with |e| = rho, and alpha >= 1/20 needs rho^2 <= 2 ln(20 opacity); 25 % of rho,
+// 0.5 |n4| and 1e-4 w4 cover its rounding.
+template <int RW, int CLS, int ROWS_USED>
+__device__ __forceinline__ uint32_t reached_groups(const float4 P1, const float4 P2, const float4 P4, float opacity,
+                                                   float ox, float oy, int row0, uint32_t valid, float& zmin) {
+    using G = GroupShape<RW, CLS>;
+    constexpr float fS = static_cast<float>(G::S);
+    zmin = -3.402823466e+38f;
+    const float rc = 2.0f * __logf(opacity * kMinAlphaRcp);
+    if (rc < 0.0f) return 0u;  // alpha <= opacity < 1/255 everywhere
+    const float3 n4 = xyz(P4);
+    const float nn = dot(n4, n4);
+    if (!(P4.w > 0.0f) || !(rc > 0.0f) || !(P4.w * P4.w - rc * nn > 0.0f)) return valid;
+    Conic q;
+    const bool ell = cutoff_conic(P1, P2, P4, opacity, q) && q.det > 1e-3f * (4.0f * q.A * q.C) && q.A < 1e30f &&
+                     q.C < 1e30f && q.det < 1e30f && q.A > 1e-30f && q.C > 1e-30f && q.det > 1e-30f;
+    if (!(q.F0 < -1e-28f)) return valid;
+    uint32_t m = 0u;
+    if (ell) {
+        const float idet = rcp_approx(q.det), i2a = 0.5f * rcp_approx(q.A), i2c = 0.5f * rcp_approx(q.C);
+        const float xc = (q.B * q.E - 2.0f * q.C * q.D) * idet, yc = (q.B * q.D - 2.0f * q.A * q.E) * idet;
+        const float Fc = -(q.F0 + 0.5f * (q.D * xc + q.E * yc));  // >= -F0 > 0
+        const float ymax = sqrt_approx(4.0f * q.A * Fc * idet), xmax = sqrt_approx(4.0f * q.C * Fc * idet);
+        const float iy = rcp_approx(ymax);
+        const float hx = sqrt_approx(2.0f * Fc * i2a), slope = -q.B * i2a;
+        const float ystar = -q.B * i2c * xmax;  // where the right extreme x = xmax lies
+        const float X = q.x0 + xc - ox, Y = q.y0 + yc - oy;  // centre relative to the tile
+        constexpr float pitch = static_cast<float>(G::GW * G::S), width = static_cast<float>((G::GW - 1) * G::S);
+        constexpr float ipitch = 1.0f / pitch;
+#pragma unroll
+        for (int i = 0; i < ROWS_USED; ++i) {
+            const int r = row0 + i;
+            const float Y0 = static_cast<float>(r * G::GH) * fS - Y - kCullPixelMargin;
+            const float Y1 = Y0 + static_cast<float>(G::GH - 1) * fS + 2.0f * kCullPixelMargin;
+            const float a = fmaxf(Y0, -ymax), e = fminf(Y1, ymax);
+            const float ta = a * iy, te = e * iy;
+            const float ha = hx * sqrt_approx(fmaxf(1.0f - ta * ta, 0.0f)), he = hx * sqrt_approx(fmaxf(1.0f - te * te, 0.0f));
+            const float R = ystar >= a && ystar <= e ? xmax : fmaxf(slope * a + ha, slope * e + he);
+            const float L = -ystar >= a && -ystar <= e ? -xmax : fminf(slope * a - ha, slope * e - he);
+            // columns whose samples [c pitch, c pitch + width] meet [X + L, X + R]
+            const int c0 = max(0, __float2int_ru(fmaxf((X + L - kCullPixelMargin - width) * ipitch, -1.0f)));
+            const int c1 = min(G::COLS - 1, __float2int_rd(fminf((X + R + kCullPixelMargin) * ipitch, 32.0f)));
+            if (a <= e && c0 <= c1) m |= ((2u << c1) - (1u << c0)) << (r * G::COLS);
+        }
+        const float rho2 = rc - 5.0912624f;  // 2 ln(20 opacity) = rc - 2 ln(255 / 20)
+        if (rho2 < -0.01f) zmin = 3.402823466e+38f;  // opacity < 1/20: no core fragment
+        else
+            zmin = P4.w - (1.25f * sqrt_approx(fmaxf(rho2, 0.0f)) + 0.5f) * sqrt_approx(nn) - 1e-4f * P4.w;
+        return m & valid;
+    }
+    float4 box;
+    bool never;
+    if (!cutoff_box(P1, P2, P4, opacity, box, never)) return valid;
+    if (never) return 0u;
+    for (int g = 0; g < G::COLS * G::ROWS; ++g) {
+        const float ax0 = ox + static_cast<float>((g % G::COLS) * G::GW) * fS, ax1 = ax0 + static_cast<float>(G::GW - 1) * fS;
+        const float ay0 = oy + static_cast<float>((g / G::COLS) * G::GH) * fS, ay1 = ay0 + static_cast<float>(G::GH - 1) * fS;
+        if (box.y >= ax0 && box.x <= ax1 && box.w >= ay0 && box.z <= ay1) m |= 1u << g;
+    }
+    return m & valid;
+}
 
+// Shared memory of a blend block: staged Gaussian records (the three VPMT rows, rgba, the core
+// depth bound), each Gaussian's group mask, and each group's list of staged slots (byte offsets
+// into the record arrays).  Slot kBlendDummy is a Gaussian of opacity 0: it pads the lists of a
+// warp's four groups to equal length.
+constexpr int kBlendThreads = 128;
+constexpr int kBlendWarps = kBlendThreads / 32;
+constexpr int kBlendGroups = 4 * kBlendWarps;
+constexpr int kBlendSlots = 2 * kBlendThreads;  // staged Gaussians: two per thread
+constexpr int kBlendDummy = kBlendSlots;
 struct BlendSmem {
-    float4* p1;
-    float4* p2;
-    float4* p4;
-    float4* rgba;
-    uint32_t* mask;
-    uint8_t (*list)[256];
+    float4 p1[kBlendSlots + 1], p2[kBlendSlots + 1], p4[kBlendSlots + 1], rgba[kBlendSlots + 1];
+    float zmin[kBlendSlots + 1];
+    uint16_t mask[kBlendSlots];
+    uint16_t list[kBlendGroups][kBlendSlots + 2];  // + 2: the groups' rows start in different banks
+    int item;
 };
+
+__device__ __forceinline__ void blend_smem_init(BlendSmem& sm) {
+    if (threadIdx.x == 0) {  // nx = (1, 0, 0), ny = (0, 1, 0): rho = 0, alpha = 0
+        sm.p1[kBlendDummy] = make_float4(1.0f, 0.0f, 0.0f, 0.0f);
+        sm.p2[kBlendDummy] = make_float4(0.0f, 1.0f, 0.0f, 0.0f);
+        sm.p4[kBlendDummy] = sm.rgba[kBlendDummy] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        sm.zmin[kBlendDummy] = 3.402823466e+38f;
+    }
+    __syncthreads();
+}
 
 // A segment of a split tile's list (SEG instantiations only).  SEG 1, the records mode: mode 0,
 // the whole list, resolved as usual (a split tile blended whole); mode 1, the first segment, whose
@@ -1713,7 +1932,7 @@ struct BlendSmem {
 // empty K-buffer: every fragment that enters it is recorded (depth, premultiplied colour) instead
 // of being blended, and the tail holds only the fragments that never entered it.  SEG 3, the exact
 // split: the segment is walked without a K-buffer and every pair is logged (`recs` = the steps a
-// warp can take, the log's stride).
+// group can take, the log's stride).
 struct SegWalk {
     uint32_t s, S;
     int mode;
@@ -1721,8 +1940,58 @@ struct SegWalk {
     char* scratch;
 };
 
-// Resolves one pixel from its K-buffer, tail and tail transmittance: the split blend's merge
-// (the same steps as the end of blend_tile).
+// The blend's per-pair arithmetic with the fused multiply-adds written out (the compiler's own
+// choice for the plain expressions, established on random pairs in both math flavours), so that
+// it does not depend on the code around it.
+__device__ __forceinline__ float mulsub(float a, float b, float c, float d) { return __fmaf_rn(a, b, -__fmul_rn(c, d)); }
+__device__ __forceinline__ float dot_xyz(const float3 a, const float3 b) {
+    return __fmaf_rn(a.z, b.z, __fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)));
+}
+__device__ __forceinline__ float3 cross_fma(const float3 a, const float3 b) {
+    return make_float3(mulsub(a.y, b.z, a.z, b.y), mulsub(a.z, b.x, a.x, b.z), mulsub(a.x, b.y, a.y, b.x));
+}
+
+// Two floats in one register pair, for the packed FP32 instructions (each half is the scalar
+// operation, rounded alike; in the flush-to-zero flavour they flush alike).
+#ifndef FHTGS_FTZ
+#define FHTGS_FTZ ""
+#endif
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 both(float a) { return pair(a, a); }
+__device__ __forceinline__ void unpair(f32x2 p, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn" FHTGS_FTZ ".f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn" FHTGS_FTZ ".f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// Inserts a fragment that is nearer than the core's last one into the sorted core, after the
+// entries of equal depth; returns the colour of the fragment that leaves it.  The selections are
+// written as such: the lanes of a warp insert at different places, and branches on them (which
+// the compiler makes of the plain loop) cost 281 instead of about 70 instructions at K = 8.
+template <int K>
+__device__ __forceinline__ uint32_t core_insert(Frag (&core)[K], float depth, const float4 pm) {
+    uint32_t color = pack_rgba(pm);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        asm("{\n .reg .pred p;\n .reg .b32 c;\n .reg .f32 d;\n setp.lt.f32 p, %0, %2;\n selp.b32 c, %3, %1, p;\n"
+            " selp.b32 %3, %1, %3, p;\n max.f32 d, %0, %2;\n min.f32 %2, %0, %2;\n mov.b32 %0, d;\n mov.b32 %1, c;\n}"
+            : "+f"(depth), "+r"(color), "+f"(core[k].depth), "+r"(core[k].color));
+    }
+    return color;
+}
+
+// Resolves one pixel from its K-buffer, tail and tail transmittance.
 template <int K>
 __device__ __forceinline__ void blend_resolve(const FrameParams& fp, const ViewParams& vp, const Frag (&core)[K],
                                               const float4 tail, const float tail_T, float pixel_x, float pixel_y,
@@ -1750,313 +2019,363 @@ __device__ __forceinline__ void blend_resolve(const FrameParams& fp, const ViewP
               __saturatef(rgb.z));
 }
 
-// Renders one 16x16 work item with the whole 256-thread block: CLS 0 a full-resolution tile with
-// its 8 warps (each RW x 32/RW pixels: 8 x 4 laid out 2 x 4, 16 x 2 stacked, or 4 x 8 laid out
-// 4 x 2); CLS 1 a periphery tile sampled at stride 2 with warps 0-1 (each min(RW, 8) wide); CLS 2
-// a ring-mode quarter tile sampled at stride 4 with lanes 0-15 of warp 0.  The Gaussians of the
-// tile's list are staged in shared memory 256 at a time; each thread culls one of them against
-// the warp rectangles, and every warp then walks only its own compacted list, in list order.
-// The warp shape only changes which pairs are culled (pairs that cannot pass the alpha test),
-// never a pixel's arithmetic.  The tile layout is a compile-time constant of each class.
-template <int K, int RW, int CLS, int SEG = 0>
-__device__ __forceinline__ void blend_tile(const FrameParams& fp, const FrameBuffers& fb, uint32_t packed,
-                                        const BlendSmem& sm, const SegWalk sw = SegWalk{0u, 1u, 0, 0, nullptr}) {
-    constexpr int NT = 256;
-    constexpr int NW = NT / 32;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+// The tile and the pixels of this thread (GroupShape).
+struct TilePixels {
+    int v;
+    uint32_t lt;
+    bool is_fovea;
+    int ox, oy, x, y[2];
+};
+template <int RW, int CLS, int PX>
+__device__ __forceinline__ TilePixels tile_pixels(const FrameParams& fp, const FrameBuffers& fb, uint32_t packed, int half) {
+    using G = GroupShape<RW, CLS>;
+    constexpr int LPG = 16 / PX, GPW = 32 / LPG;  // lanes per group, groups per warp
+    TilePixels tp;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k = lane % LPG;
+    const int group = CLS == 0 ? half * kBlendWarps * GPW + GPW * warp + lane / LPG : CLS == 1 ? lane / LPG : 0;
+    tp.v = item_view(packed);
+    const uint32_t item = item_index(packed);
+    const ViewParams& vp = fb.views[tp.v];
+    tp.lt = (CLS != 0 ? fb.work_low : fb.work_full)[static_cast<size_t>(tp.v) * fp.max_large + item];
+    tp.is_fovea = CLS == 0 && item < fb.status[tp.v].n_fovea_large;
+    tp.ox = static_cast<int>(tp.lt % static_cast<uint32_t>(vp.glw)) * kTileLarge;
+    tp.oy = static_cast<int>(tp.lt / static_cast<uint32_t>(vp.glw)) * kTileLarge;
+    tp.x = tp.ox + ((group % G::COLS) * G::GW + k % G::GW) * G::S;
+    tp.y[0] = tp.oy + ((group / G::COLS) * G::GH + k / G::GW) * G::S;
+    tp.y[1] = tp.y[0] + G::GH / 2 * G::S;
+    return tp;
+}
+
+// Blends one tile, or half of one (PX 1: `half`), with a team of threads: the block (CLS 0), a
+// warp (CLS 1) or 8 lanes (CLS 2; `live` false: no tile for this group).  The team stages its tile's list two
+// Gaussians a thread at a time; every thread culls its two against the tile's sample groups, each
+// group's survivors become its list, and the warp walks its groups' lists side by side, in list
+// order.  Which pairs are culled (pairs that cannot pass the alpha test) never changes a
+// pixel's arithmetic.
+template <int K, int RW, int CLS, int PX, int SEG = 0>
+__device__ __forceinline__ void blend_tile(const FrameParams& fp, const FrameBuffers& fb, uint32_t packed, int half, bool live,
+                                           BlendSmem& sm, const SegWalk sw = SegWalk{0u, 1u, 0, 0, nullptr}) {
+    using G = GroupShape<RW, CLS>;
+    constexpr uint32_t TEAM = CLS == 0 ? kBlendThreads : CLS == 1 ? 32 : 8;
+    constexpr uint32_t BATCH = 2 * TEAM;
+    constexpr bool log_mode = SEG == 3;  // the exact split's segment: log the fragments only
+    constexpr int NT = kSplitPx;
+    constexpr int LPG = 16 / PX, GPW = 32 / LPG;  // lanes per group, groups per warp
+    static_assert(PX == 2 || (CLS == 0 && SEG == 0), "half items are full-resolution");
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, grp = lane / LPG;
+    const uint32_t team_tid = CLS == 0 ? tid : CLS == 1 ? lane : lane & 7;
+    const uint32_t team_base = CLS == 0 ? 0u : CLS == 1 ? warp * BATCH : (warp * 4 + grp) * BATCH;
     const uint32_t lanemask_lt = (1u << lane) - 1u;
-    const int v = static_cast<int>(packed >> 24);
-    const int item = static_cast<int>(packed & (kItemLowres - 1u));
-    const ViewParams& vp = fb.views[v];
-    const FrameStatus& st = fb.status[v];
-    const uint32_t lt = CLS != 0 ? fb.work_low[static_cast<size_t>(v) * fp.max_large + item]
-                            : fb.work_full[static_cast<size_t>(v) * fp.max_large + item];
-    const bool is_fovea = CLS == 0 && static_cast<uint32_t>(item) < st.n_fovea_large;
-    constexpr int S = CLS == 0 ? 1 : CLS == 1 ? kStride : kQuarterStride;
-    // warp rectangle rw x rh (powers of two); warps laid out 2^wx_bits per row
-    constexpr int RW_LOW = RW > 8 ? 8 : RW;  // the periphery sample grid is 8 wide
-    constexpr int RW_BITS = RW == 4 ? 2 : RW == 8 ? 3 : 4, RW_LOW_BITS = RW_LOW == 4 ? 2 : 3;
-    constexpr int rw_bits = CLS == 2 ? 2 : CLS == 1 ? RW_LOW_BITS : RW_BITS;
-    constexpr int rw = 1 << rw_bits, rh = 32 >> rw_bits;
-    constexpr int rh_used = CLS == 2 ? 4 : rh;  // sample rows of a warp that lie in the tile
-    constexpr int wx_bits = CLS == 2 ? 0 : (CLS == 1 ? 3 : 4) - rw_bits;
-    constexpr int n_warps = CLS == 2 ? 1 : CLS == 1 ? 2 : NW;
-    const int ox = static_cast<int>(lt % static_cast<uint32_t>(vp.glw)) * kTileLarge;
-    const int oy = static_cast<int>(lt / static_cast<uint32_t>(vp.glw)) * kTileLarge;
-    const int lx = (warp & ((1 << wx_bits) - 1)) * rw + (lane & (rw - 1));
-    const int ly = (warp >> wx_bits) * rh + (lane >> rw_bits);
-    const int px_i = ox + lx * S, py_i = oy + ly * S;
-    const bool inside = warp < n_warps && (lane >> rw_bits) < rh_used && px_i < vp.width && py_i < vp.height;
-    const float pixel_x = __uint2float_rn(static_cast<uint32_t>(px_i));
-    const float pixel_y = __uint2float_rn(static_cast<uint32_t>(py_i));
-    uint2 range = fb.ranges[static_cast<size_t>(v) * fp.max_large + lt];
+    const TilePixels pp = tile_pixels<RW, CLS, PX>(fp, fb, packed, half);
+    const ViewParams& vp = fb.views[pp.v];
+    const float pixel_x = __uint2float_rn(static_cast<uint32_t>(pp.x));
+    float pixel_y[PX];
+#pragma unroll
+    for (int i = 0; i < PX; ++i) pixel_y[i] = __uint2float_rn(static_cast<uint32_t>(pp.y[i]));
+    const f32x2 npixel_y = pair(-pixel_y[0], -pixel_y[PX - 1]);
+    constexpr int ROWS_USED = CLS == 0 ? G::ROWS * PX / 2 : G::ROWS;
+    const int row0 = half * ROWS_USED;
+    uint32_t valid = 0u;  // this item's groups with a pixel inside the image
+#pragma unroll
+    for (int i = 0; i < G::COLS * ROWS_USED; ++i) {
+        const int g = row0 * G::COLS + i;
+        if (pp.ox + (g % G::COLS) * G::GW * G::S < vp.width && pp.oy + (g / G::COLS) * G::GH * G::S < vp.height) valid |= 1u << g;
+    }
+    uint2 range = live ? fb.ranges[static_cast<size_t>(pp.v) * fp.max_large + pp.lt] : make_uint2(0u, 0u);
     if constexpr (SEG != 0) {  // segment s of S equal parts of the list
         const uint64_t len = range.y > range.x ? range.y - range.x : 0u;
         const uint32_t lo = range.x + static_cast<uint32_t>(len * sw.s / sw.S);
         const uint32_t hi = range.x + static_cast<uint32_t>(len * (sw.s + 1u) / sw.S);
         range = make_uint2(lo, hi);
     }
-    const uint32_t* vals = fb.vals[fb.final_buf] + static_cast<size_t>(v) * fp.cap;
-    const float4* rec = fb.rec + 4 * static_cast<size_t>(v) * fp.n_prims;
-    uint32_t n_rec = 0;     // SEG mode 2: fragments that entered the K-buffer
-    uint32_t n_logged = 0;  // SEG mode 3: steps of this warp logged so far
-    constexpr bool log_mode = SEG == 3;  // the exact split's segment: log the fragments only
+    const uint32_t* vals = fb.vals[fb.final_buf] + static_cast<size_t>(pp.v) * fp.cap;
+    const float4* rec = fb.rec + 4 * static_cast<size_t>(pp.v) * fp.n_prims;
+    uint32_t n_rec[PX] = {};     // SEG mode 2: fragments that entered the K-buffer
+    uint32_t n_logged[GPW] = {}; // SEG mode 3: steps of this warp's groups logged so far
 
-    float tail_T = 1.0f;
-    float4 tail = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    Frag core[K];
+    float tail_T[PX];
+    float4 tail[PX];
+    Frag core[PX][K];
 #pragma unroll
-    for (int k = 0; k < K; ++k) { core[k].depth = 3.402823466e+38f; core[k].color = 0u; }
+    for (int i = 0; i < PX; ++i) {
+        tail_T[i] = 1.0f;
+        tail[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int k = 0; k < K; ++k) { core[i][k].depth = 3.402823466e+38f; core[i][k].color = 0u; }
+    }
 
-    for (uint32_t start = range.x; start < range.y; start += NT) {
-        const uint32_t n_batch = min(static_cast<uint32_t>(NT), range.y - start);
-        __syncthreads();
-        if (static_cast<uint32_t>(tid) < n_batch && vals[start + tid] >= static_cast<uint32_t>(fp.n_prims)) {
-            sm.mask[tid] = 0u;  // a sentinel slot: no primitive to blend
-        } else if (static_cast<uint32_t>(tid) < n_batch) {
-            const uint32_t p = vals[start + tid];
-            const float4* r = rec + 4 * static_cast<size_t>(p);
-            const float4 P1 = r[0], P2 = r[1], P4 = r[2], c = r[3];
-            sm.p1[tid] = P1;
-            sm.p2[tid] = P2;
-            sm.p4[tid] = P4;
-            sm.rgba[tid] = c;
-            float4 box;
-            bool never;
-            uint32_t m = (1u << n_warps) - 1u;
-            if (cutoff_box(P1, P2, P4, c.w, box, never)) {
-                if (never) m = 0u;
-                else {
-                    Conic q;
-                    const bool ell = cutoff_conic(P1, P2, P4, c.w, q);
-                    m = 0u;
-                    for (int w = 0; w < n_warps; ++w) {
-                        const float ax0 = static_cast<float>(ox + (w & ((1 << wx_bits) - 1)) * rw * S);
-                        const float ax1 = ax0 + static_cast<float>((rw - 1) * S);
-                        const float ay0 = static_cast<float>(oy + (w >> wx_bits) * rh * S);
-                        const float ay1 = ay0 + static_cast<float>((rh_used - 1) * S);
-                        if (box.y >= ax0 && box.x <= ax1 && box.w >= ay0 && box.z <= ay1 &&
-                            (!ell || conic_meets_rect(q, ax0, ax1, ay0, ay1)))
-                            m |= 1u << w;
-                    }
-                }
+    for (uint32_t start = range.x; CLS == 2 ? __any_sync(0xffffffffu, start < range.y) : start < range.y; start += BATCH) {
+        const uint32_t n_batch = start < range.y ? min(BATCH, range.y - start) : 0u;
+        if (CLS == 0) __syncthreads(); else __syncwarp();
+        uint32_t mask[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t i = h * TEAM + team_tid, slot = team_base + i;
+            mask[h] = 0u;
+            const uint32_t p = i < n_batch ? vals[start + i] : kNoPrimitive;
+            if (p < static_cast<uint32_t>(fp.n_prims)) {  // (sentinel slots hold no primitive)
+                const float4* r = rec + 4 * static_cast<size_t>(p);
+                const float4 P1 = r[0], P2 = r[1], P4 = r[2], c = r[3];
+                sm.p1[slot] = P1;
+                sm.p2[slot] = P2;
+                sm.p4[slot] = P4;
+                sm.rgba[slot] = c;
+                mask[h] = reached_groups<RW, CLS, ROWS_USED>(P1, P2, P4, c.w, static_cast<float>(pp.ox),
+                                                             static_cast<float>(pp.oy), row0, valid, sm.zmin[slot]);
             }
-            sm.mask[tid] = m;
+            if (CLS != 2) sm.mask[slot] = static_cast<uint16_t>(mask[h]);
         }
-        __syncthreads();
-        // this warp's list: the batch positions whose mask has its bit, in order
-        int n_mine = 0;
-        for (uint32_t c0 = 0; c0 < n_batch; c0 += 32) {
-            const uint32_t j = c0 + lane;
-            const bool hit = j < n_batch && ((sm.mask[j] >> warp) & 1u);
-            const uint32_t b = __ballot_sync(0xffffffffu, hit);
-            if (hit) sm.list[warp][n_mine + __popc(b & lanemask_lt)] = static_cast<uint8_t>(j);
-            if constexpr (log_mode) {
-                if (hit)  // each step's Gaussian colour and opacity
-                    reinterpret_cast<float4*>(sw.scratch + 256u * split_log_pos_unit())
-                        [static_cast<uint32_t>(warp) * sw.recs + n_logged + n_mine + __popc(b & lanemask_lt)] = sm.rgba[j];
-            }
-            n_mine += __popc(b);
-        }
-        __syncwarp();
+        if (CLS == 0) __syncthreads(); else __syncwarp();
+        // the lists of this warp's groups: the staged slots whose mask has the group's bit
+        uint32_t n_mine, n_max;
         uint32_t step0 = 0;
-        if constexpr (SEG != 0) {
-            step0 = n_logged;
-            n_logged += static_cast<uint32_t>(n_mine);
-        }
-        if (!inside) continue;
-        for (int t = 0; t < n_mine; ++t) {
-            const int j = sm.list[warp][t];
-            const float4 VPMT1 = sm.p1[j], VPMT2 = sm.p2[j], VPMT4 = sm.p4[j];
-            const float4 plane_x = VPMT1 - VPMT4 * pixel_x;
-            const float4 plane_y = VPMT2 - VPMT4 * pixel_y;
-            const float3 nx = xyz(plane_x), ny = xyz(plane_y);
-            const float3 m = plane_x.w * ny - nx * plane_y.w;
-            const float3 d = cross(nx, ny);
-            const float num = dot(m, m);
-            const float den = dot(d, d);
-            // In almost every warp step some lane passes both tests, so the fragment is
-            // evaluated for every lane and the tests only gate its effects (no divergent
-            // exits; a lane that failed cannot contribute: its `frag` is false whatever
-            // rcp/exp return for it).
-            const bool live = !(num > kMaxCutoffSq * den);
-            const float den_rcp = 1.0f / den;
-            const float G = expf(-0.5f * num * den_rcp);
-            const float4 c = sm.rgba[j];
-            const float alpha = fminf(c.w * G, kMaxFragmentAlpha);
-            const bool frag = live && !(alpha < kMinAlpha);
-            float4 pm = make_float4(c.x * alpha, c.y * alpha, c.z * alpha, alpha);
-            // the depth matters only to a fragment that may enter the core (alpha >= 1/20):
-            // evaluated when some lane of the warp has such a fragment (a warp-uniform branch,
-            // so that warps whose fragments are all faint skip it without reconvergence work)
-            const bool cand = frag && alpha >= kMinAlphaCore;
-            float logged_depth = 0.0f;
-            if (__any_sync(__activemask(), cand)) {
-                const float3 ep = cross(d, m) * den_rcp;
-                const float depth = dot(xyz(VPMT4), ep) + VPMT4.w;
-                if constexpr (log_mode) logged_depth = depth;
-                if (cand && depth < core[K - 1].depth && !log_mode) {
-                    if constexpr (SEG == 1) {
-                        if (sw.mode == 2) {  // recorded; the merge decides what it does
-                            if (n_rec < static_cast<uint32_t>(sw.recs)) {
-                                reinterpret_cast<float*>(sw.scratch + 6 * 4 * NT)[n_rec * NT + tid] = depth;
-                                reinterpret_cast<float4*>(sw.scratch + (6 + sw.recs) * 4 * NT)[n_rec * NT + tid] = pm;
-                            }
-                            ++n_rec;
-                        }
-                    }
-                    Frag f;
-                    f.depth = depth;
-                    f.color = pack_rgba(pm);
+        if constexpr (CLS != 2) {
+            uint32_t n[GPW] = {};
+            for (uint32_t c0 = 0; c0 < n_batch; c0 += 32) {
+                const uint32_t slot = team_base + c0 + lane;
+                const uint32_t mk = sm.mask[slot] >> (CLS == 0 ? (half * kBlendWarps + warp) * GPW : 0);
 #pragma unroll
-                    for (int k = 0; k < K; ++k) {
-                        if (f.depth < core[k].depth) {
-                            const Frag tf = core[k];
-                            core[k] = f;
-                            f = tf;
+                for (int g = 0; g < GPW; ++g) {
+                    const bool hit = (mk >> g) & 1u;
+                    const uint32_t b = __ballot_sync(0xffffffffu, hit);
+                    const uint32_t at = n[g] + __popc(b & lanemask_lt);
+                    if (hit) {
+                        sm.list[GPW * warp + g][at] = static_cast<uint16_t>(slot * 16u);
+                        if constexpr (log_mode)  // each step's Gaussian colour and opacity
+                            reinterpret_cast<float4*>(sw.scratch + 256u * split_log_pos_unit())
+                                [static_cast<uint32_t>(GPW * warp + g) * sw.recs + n_logged[g] + at] = sm.rgba[slot];
+                    }
+                    n[g] += __popc(b);
+                }
+            }
+            n_max = n_mine = n[0];
+            step0 = n_logged[0];
+#pragma unroll
+            for (int g = 0; g < GPW; ++g) {
+                n_max = max(n_max, n[g]);
+                if (grp == g) n_mine = n[g];
+                if (grp == g) step0 = n_logged[g];
+                n_logged[g] += n[g];
+            }
+        } else {
+            const uint32_t b0 = (__ballot_sync(0xffffffffu, mask[0] != 0u) >> (8 * grp)) & 0xffu;
+            const uint32_t b1 = (__ballot_sync(0xffffffffu, mask[1] != 0u) >> (8 * grp)) & 0xffu;
+            const uint32_t lt8 = (1u << (lane & 7)) - 1u;
+            uint16_t* list = sm.list[GPW * warp + grp];
+            if (mask[0]) list[__popc(b0 & lt8)] = static_cast<uint16_t>((team_base + team_tid) * 16u);
+            if (mask[1]) list[__popc(b0) + __popc(b1 & lt8)] = static_cast<uint16_t>((team_base + TEAM + team_tid) * 16u);
+            n_mine = __popc(b0) + __popc(b1);
+            n_max = __reduce_max_sync(0xffffffffu, n_mine);
+        }
+        uint16_t* list = sm.list[GPW * warp + grp];
+        for (uint32_t t = n_mine + lane % LPG; t < n_max; t += LPG) list[t] = kBlendDummy * 16;
+        __syncwarp();
+        for (uint32_t t = 0; t < n_max; ++t) {
+            const uint32_t off = list[t];
+            auto lds = [&](const float4* a) { return *reinterpret_cast<const float4*>(reinterpret_cast<const char*>(a) + off); };
+            const float4 A = lds(sm.p1), B = lds(sm.p2), C = lds(sm.p4), c = lds(sm.rgba);
+            const float zmin = *reinterpret_cast<const float*>(reinterpret_cast<const char*>(sm.zmin) + (off >> 2));
+            float3 m[PX], d[PX];
+            float rcp[PX], alpha[PX];
+            float4 pm[PX];
+            bool frag[PX], cand = false;
+            // the fragment is evaluated for every lane and the tests only gate its effects (no
+            // divergent exits; a lane that failed cannot contribute, whatever rcp / exp return)
+            if constexpr (PX == 2) {
+                // both pixels in packed arithmetic: m and d are the negatives of the scalar form's,
+                // (-a) b + (c d) for a b - (c d), which leaves num, den and cross(d, m) the same
+                const f32x2 X = both(__fmaf_rn(-C.x, pixel_x, A.x)), Y = both(__fmaf_rn(-C.y, pixel_x, A.y)),
+                            Z = both(__fmaf_rn(-C.z, pixel_x, A.z)), nX = both(__fmaf_rn(C.x, pixel_x, -A.x)),
+                            nY = both(__fmaf_rn(C.y, pixel_x, -A.y)), nZ = both(__fmaf_rn(C.z, pixel_x, -A.z)),
+                            nW = both(__fmaf_rn(C.w, pixel_x, -A.w));
+                const f32x2 yx = fma2(both(C.x), npixel_y, both(B.x)), yy = fma2(both(C.y), npixel_y, both(B.y)),
+                            yz = fma2(both(C.z), npixel_y, both(B.z)), yw = fma2(both(C.w), npixel_y, both(B.w));
+                const f32x2 mx = fma2(nW, yx, mul2(X, yw)), my = fma2(nW, yy, mul2(Y, yw)), mz = fma2(nW, yz, mul2(Z, yw));
+                const f32x2 dx = fma2(nY, yz, mul2(Z, yy)), dy = fma2(nZ, yx, mul2(X, yz)), dz = fma2(nX, yy, mul2(Y, yx));
+                const f32x2 num2 = fma2(mz, mz, fma2(mx, mx, mul2(my, my))), den2 = fma2(dz, dz, fma2(dx, dx, mul2(dy, dy)));
+                float num[2], den[2], lim[2], e[2];
+                unpair(num2, num[0], num[1]);
+                unpair(den2, den[0], den[1]);
+                unpair(mul2(both(kMaxCutoffSq), den2), lim[0], lim[1]);
+                rcp[0] = 1.0f / den[0];
+                rcp[1] = 1.0f / den[1];
+                unpair(mul2(mul2(both(-0.5f), num2), pair(rcp[0], rcp[1])), e[0], e[1]);
+                unpair(mul2(both(c.w), pair(expf(e[0]), expf(e[1]))), alpha[0], alpha[1]);
+                alpha[0] = fminf(alpha[0], kMaxFragmentAlpha);
+                alpha[1] = fminf(alpha[1], kMaxFragmentAlpha);
+                const f32x2 al = pair(alpha[0], alpha[1]);
+                unpair(mul2(both(c.x), al), pm[0].x, pm[1].x);
+                unpair(mul2(both(c.y), al), pm[0].y, pm[1].y);
+                unpair(mul2(both(c.z), al), pm[0].z, pm[1].z);
+                unpair(mx, m[0].x, m[1].x);
+                unpair(my, m[0].y, m[1].y);
+                unpair(mz, m[0].z, m[1].z);
+                unpair(dx, d[0].x, d[1].x);
+                unpair(dy, d[0].y, d[1].y);
+                unpair(dz, d[0].z, d[1].z);
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    pm[i].w = alpha[i];
+                    frag[i] = !(num[i] > lim[i]) && !(alpha[i] < kMinAlpha);
+                    cand = cand || (frag[i] && (log_mode || zmin < core[i][K - 1].depth));
+                }
+            } else {
+                const float3 nx = make_float3(__fmaf_rn(-C.x, pixel_x, A.x), __fmaf_rn(-C.y, pixel_x, A.y), __fmaf_rn(-C.z, pixel_x, A.z));
+                const float wx = __fmaf_rn(-C.w, pixel_x, A.w);
+                const float3 ny = make_float3(__fmaf_rn(-C.x, pixel_y[0], B.x), __fmaf_rn(-C.y, pixel_y[0], B.y),
+                                              __fmaf_rn(-C.z, pixel_y[0], B.z));
+                const float wy = __fmaf_rn(-C.w, pixel_y[0], B.w);
+                m[0] = make_float3(mulsub(wx, ny.x, nx.x, wy), mulsub(wx, ny.y, nx.y, wy), mulsub(wx, ny.z, nx.z, wy));
+                d[0] = cross_fma(nx, ny);
+                const float num = dot_xyz(m[0], m[0]), den = dot_xyz(d[0], d[0]);
+                const bool in = !(num > kMaxCutoffSq * den);
+                rcp[0] = 1.0f / den;
+                alpha[0] = fminf(c.w * expf(-0.5f * num * rcp[0]), kMaxFragmentAlpha);
+                frag[0] = in && !(alpha[0] < kMinAlpha);
+                cand = frag[0] && zmin < core[0][K - 1].depth;
+                pm[0] = make_float4(c.x * alpha[0], c.y * alpha[0], c.z * alpha[0], alpha[0]);
+            }
+            // The depth matters only to a fragment that may enter the core: alpha >= 1/20 and a
+            // depth below the core's last.  `zmin` bounds it from below, so that once the near
+            // Gaussians are in, almost no step evaluates it (a warp-uniform branch).
+            float logged_depth[PX] = {};
+            if (__any_sync(0xffffffffu, cand)) {
+#pragma unroll
+                for (int i = 0; i < PX; ++i) {
+                    const float3 e = cross_fma(d[i], m[i]);
+                    const float3 ep = make_float3(__fmul_rn(e.x, rcp[i]), __fmul_rn(e.y, rcp[i]), __fmul_rn(e.z, rcp[i]));
+                    const float depth = __fadd_rn(dot_xyz(xyz(C), ep), C.w);
+                    if constexpr (log_mode) logged_depth[i] = depth;
+                    if constexpr (!log_mode) {
+                        const bool ins = frag[i] && alpha[i] >= kMinAlphaCore && depth < core[i][K - 1].depth;
+                        if (__any_sync(0xffffffffu, ins)) {  // lanes without an insertion: FLT_MAX changes nothing
+                            if constexpr (SEG == 1) {
+                                if (ins && sw.mode == 2) {  // recorded; the merge decides what it does
+                                    if (n_rec[i] < static_cast<uint32_t>(sw.recs)) {
+                                        const uint32_t at = n_rec[i] * NT + tid + i * kBlendThreads;
+                                        reinterpret_cast<float*>(sw.scratch + 6 * 4 * NT)[at] = depth;
+                                        reinterpret_cast<float4*>(sw.scratch + (6 + sw.recs) * 4 * NT)[at] = pm[i];
+                                    }
+                                    ++n_rec[i];
+                                }
+                            }
+                            float4 ev = unpack_rgba(core_insert<K>(core[i], ins ? depth : 3.402823466e+38f, pm[i]));
+                            if constexpr (SEG == 1) {
+                                if (sw.mode == 2) ev = make_float4(0.0f, 0.0f, 0.0f, 0.0f);  // adds nothing below
+                            }
+                            pm[i] = make_float4(ins ? ev.x : pm[i].x, ins ? ev.y : pm[i].y, ins ? ev.z : pm[i].z,
+                                                ins ? ev.w : pm[i].w);
                         }
                     }
-                    pm = unpack_rgba(f.color);
-                    if constexpr (SEG == 1) {
-                        if (sw.mode == 2) pm = make_float4(0.0f, 0.0f, 0.0f, 0.0f);  // adds nothing below
+                }
+            }
+            if constexpr (log_mode) {  // the pairs' alphas (-1: no fragment) and depths, for the replay
+                if (t < n_mine) {
+                    float2* fr = reinterpret_cast<float2*>(sw.scratch + 256u * split_log_frag_unit(sw.recs)) +
+                                 (static_cast<uint32_t>(GPW * warp + grp) * sw.recs + step0 + t) * 16u + (lane & 7);
+#pragma unroll
+                    for (int i = 0; i < PX; ++i) fr[8 * i] = make_float2(frag[i] ? alpha[i] : -1.0f, logged_depth[i]);
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < PX; ++i) {
+                    if (frag[i]) {
+                        const float pt = 1.0f - pm[i].w;
+                        tail[i] += pm[i];
+                        tail_T[i] *= pt;
                     }
                 }
-            }
-            if constexpr (log_mode) {
-                {  // the pair's alpha (-1: no fragment) and depth, for the replay
-                    reinterpret_cast<float2*>(sw.scratch + 256u * split_log_frag_unit(sw.recs))
-                        [(static_cast<uint32_t>(warp) * sw.recs + step0 + t) * 32u + lane] =
-                        make_float2(frag ? alpha : -1.0f, logged_depth);
-                    continue;
-                }
-            }
-            if (frag) {
-                const float pt = 1.0f - pm.w;
-                tail += pm;
-                tail_T *= pt;
             }
         }
     }
     if constexpr (SEG == 1) {
-        if (sw.mode == 1) {
-            float* cd = reinterpret_cast<float*>(sw.scratch);
-            uint32_t* cc = reinterpret_cast<uint32_t*>(sw.scratch + K * 4 * NT);
+        if (sw.mode != 0) {
+            // mode 1: the K-buffer, tail and transmittance; mode 2: the record count and the tail
+            const int head = sw.mode == 1 ? 2 * K : 1;
 #pragma unroll
-            for (int k = 0; k < K; ++k) {
-                cd[k * NT + tid] = core[k].depth;
-                cc[k * NT + tid] = core[k].color;
+            for (int i = 0; i < PX; ++i) {
+                const int at = tid + i * kBlendThreads;
+                if (sw.mode == 1) {
+#pragma unroll
+                    for (int k = 0; k < K; ++k) {
+                        reinterpret_cast<float*>(sw.scratch)[k * NT + at] = core[i][k].depth;
+                        reinterpret_cast<uint32_t*>(sw.scratch + K * 4 * NT)[k * NT + at] = core[i][k].color;
+                    }
+                } else {
+                    reinterpret_cast<uint32_t*>(sw.scratch)[at] = n_rec[i];
+                }
+                reinterpret_cast<float4*>(sw.scratch + head * 4 * NT)[at] = tail[i];
+                reinterpret_cast<float*>(sw.scratch + (head + 4) * 4 * NT)[at] = tail_T[i];
             }
-            reinterpret_cast<float4*>(sw.scratch + 2 * K * 4 * NT)[tid] = tail;
-            reinterpret_cast<float*>(sw.scratch + (2 * K + 4) * 4 * NT)[tid] = tail_T;
-            return;
-        }
-        if (sw.mode == 2) {
-            reinterpret_cast<uint32_t*>(sw.scratch)[tid] = n_rec;
-            reinterpret_cast<float4*>(sw.scratch + 4 * NT)[tid] = tail;
-            reinterpret_cast<float*>(sw.scratch + 5 * 4 * NT)[tid] = tail_T;
             return;
         }
     }
     if constexpr (log_mode) {
-        if (lane == 0) reinterpret_cast<uint32_t*>(sw.scratch)[warp] = n_logged;
-        return;
-    }
-    if (inside) {
-        float3 rgb = make_float3(0.0f, 0.0f, 0.0f);
-        float Tc = 1.0f;
+        if (lane < GPW) {
+            uint32_t n = n_logged[0];
 #pragma unroll
-        for (int k = 0; k < K && Tc >= kTransmittanceThreshold; ++k) {
-            const float4 c = unpack_rgba(core[k].color);
-            rgb += Tc * xyz(c);
-            Tc *= 1.0f - c.w;
+            for (int g = 1; g < GPW; ++g)
+                if (lane == g) n = n_logged[g];
+            reinterpret_cast<uint32_t*>(sw.scratch)[GPW * warp + lane] = n;
         }
-        if (Tc >= kTransmittanceThreshold && tail.w >= kMinAlpha) {
-            const float wt = Tc * (1.0f - tail_T);
-            rgb += wt * (1.0f / tail.w) * xyz(tail);
-        }
-        if (fp.bg_type != 0) {
-            const float wb = Tc * tail_T;
-            if (wb >= kTransmittanceThreshold) {
-                if (fp.bg_type == 1) rgb += wb * eval_sh_background(vp, fp.bg_data, pixel_x, pixel_y);
-                else rgb += wb * eval_tex_background(vp, fp.bg_data, fp.tex_w, fp.tex_h, fp.bg_type == 3, pixel_x, pixel_y);
-            }
-        }
-        float* out = is_fovea ? vp.image : vp.work;
-        store_rgb(out, vp.width, vp.height, px_i, py_i, fp.to_chw != 0, __saturatef(rgb.x), __saturatef(rgb.y),
-                  __saturatef(rgb.z));
+    } else {
+#pragma unroll
+        for (int i = 0; i < PX; ++i)
+            if (live && pp.x < vp.width && pp.y[i] < vp.height)
+                blend_resolve<K>(fp, vp, core[i], tail[i], tail_T[i], pixel_x, pixel_y[i], pp.is_fovea ? vp.image : vp.work,
+                                 pp.x, pp.y[i]);
     }
 }
 
 // Exact split: the merge.  Each pixel replays, segment by segment and step by step, the
-// fragments its warp evaluated, with the walk's own K-buffer insertion and tail accumulation, so
+// fragments its group evaluated, with the walk's own K-buffer insertion and tail accumulation, so
 // the operations and their order are those of the serial walk over the whole list.
 template <int K, int RW>
 __device__ __forceinline__ void split_replay(const FrameParams& fp, const FrameBuffers& fb, const SplitArgs& sp,
                                              uint32_t packed, uint32_t seg0, uint32_t S, uint32_t log_stride) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int v = static_cast<int>(packed >> 24);
-    const int item = static_cast<int>(packed & (kItemLowres - 1u));
-    const ViewParams& vp = fb.views[v];
-    const uint32_t lt = fb.work_full[static_cast<size_t>(v) * fp.max_large + item];
-    const bool is_fovea = static_cast<uint32_t>(item) < fb.status[v].n_fovea_large;
-    constexpr int rw_bits = RW == 4 ? 2 : RW == 8 ? 3 : 4;
-    constexpr int rw = 1 << rw_bits, rh = 32 >> rw_bits;
-    constexpr int wx_bits = 4 - rw_bits;
-    const int px_i = static_cast<int>(lt % static_cast<uint32_t>(vp.glw)) * kTileLarge + (warp & ((1 << wx_bits) - 1)) * rw + (lane & (rw - 1));
-    const int py_i = static_cast<int>(lt / static_cast<uint32_t>(vp.glw)) * kTileLarge + (warp >> wx_bits) * rh + (lane >> rw_bits);
-    if (px_i >= vp.width || py_i >= vp.height) return;
-    float tail_T = 1.0f;
-    float4 tail = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    Frag core[K];
-#pragma unroll
-    for (int k = 0; k < K; ++k) { core[k].depth = 3.402823466e+38f; core[k].color = 0u; }
+    const int lane = threadIdx.x & 31, group = threadIdx.x >> 3;
+    const TilePixels pp = tile_pixels<RW, 0, 2>(fp, fb, packed, 0);
+    const ViewParams& vp = fb.views[pp.v];
     constexpr uint32_t kChunk = 4;  // steps whose log entries are loaded before any is replayed
-    for (uint32_t k = 0; k < S; ++k) {
-        const char* b = sp.pool + 256ull * sp.seg_unit[seg0 + k];
-        const uint32_t n = __ldcg(reinterpret_cast<const uint32_t*>(b) + warp);
-        const float4* col = reinterpret_cast<const float4*>(b + 256u * split_log_pos_unit()) +
-                            static_cast<size_t>(warp) * log_stride;
-        const float2* fr = reinterpret_cast<const float2*>(b + 256u * split_log_frag_unit(log_stride)) +
-                           static_cast<size_t>(warp) * log_stride * 32u + lane;
-        for (uint32_t t0 = 0; t0 < n; t0 += kChunk) {
-            float2 ads[kChunk];
-            float4 cs[kChunk];
+    for (int px = 0; px < 2; ++px) {
+        const int py_i = px == 0 ? pp.y[0] : pp.y[1];
+        if (pp.x >= vp.width || py_i >= vp.height) continue;
+        float tail_T = 1.0f;
+        float4 tail = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        Frag core[K];
 #pragma unroll
-            for (uint32_t i = 0; i < kChunk; ++i) {
-                const bool ok = t0 + i < n;
-                ads[i] = ok ? __ldcg(fr + (t0 + i) * 32u) : make_float2(-1.0f, 0.0f);
-                cs[i] = ok ? __ldcg(col + t0 + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            }
+        for (int k = 0; k < K; ++k) { core[k].depth = 3.402823466e+38f; core[k].color = 0u; }
+        for (uint32_t k = 0; k < S; ++k) {
+            const char* b = sp.pool + 256ull * sp.seg_unit[seg0 + k];
+            const uint32_t n = __ldcg(reinterpret_cast<const uint32_t*>(b) + group);
+            const float4* col = reinterpret_cast<const float4*>(b + 256u * split_log_pos_unit()) +
+                                static_cast<size_t>(group) * log_stride;
+            const float2* fr = reinterpret_cast<const float2*>(b + 256u * split_log_frag_unit(log_stride)) +
+                               static_cast<size_t>(group) * log_stride * 16u + (lane & 7) + 8 * px;
+            for (uint32_t t0 = 0; t0 < n; t0 += kChunk) {
+                float2 ads[kChunk];
+                float4 cs[kChunk];
 #pragma unroll
-            for (uint32_t i = 0; i < kChunk; ++i) {
-            const float2 ad = ads[i];
-            if (ad.x < 0.0f) continue;  // not a fragment
-            const float alpha = ad.x;
-            const float4 c = cs[i];
-            float4 pm = make_float4(c.x * alpha, c.y * alpha, c.z * alpha, alpha);
-            const bool cand = alpha >= kMinAlphaCore;
-            if (cand && ad.y < core[K - 1].depth) {
-                Frag f;
-                f.depth = ad.y;
-                f.color = pack_rgba(pm);
-#pragma unroll
-                for (int q = 0; q < K; ++q) {
-                    if (f.depth < core[q].depth) {
-                        const Frag tf = core[q];
-                        core[q] = f;
-                        f = tf;
-                    }
+                for (uint32_t i = 0; i < kChunk; ++i) {
+                    const bool ok = t0 + i < n;
+                    ads[i] = ok ? __ldcg(fr + (t0 + i) * 16u) : make_float2(-1.0f, 0.0f);
+                    cs[i] = ok ? __ldcg(col + t0 + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                 }
-                pm = unpack_rgba(f.color);
-            }
-            const float pt = 1.0f - pm.w;
-            tail += pm;
-            tail_T *= pt;
+#pragma unroll
+                for (uint32_t i = 0; i < kChunk; ++i) {
+                    const float alpha = ads[i].x;
+                    if (alpha < 0.0f) continue;  // not a fragment
+                    float4 pm = make_float4(cs[i].x * alpha, cs[i].y * alpha, cs[i].z * alpha, alpha);
+                    if (alpha >= kMinAlphaCore && ads[i].y < core[K - 1].depth) pm = unpack_rgba(core_insert<K>(core, ads[i].y, pm));
+                    const float pt = 1.0f - pm.w;
+                    tail += pm;
+                    tail_T *= pt;
+                }
             }
         }
+        blend_resolve<K>(fp, vp, core, tail, tail_T, __uint2float_rn(static_cast<uint32_t>(pp.x)),
+                         __uint2float_rn(static_cast<uint32_t>(py_i)), pp.is_fovea ? vp.image : vp.work, pp.x, py_i);
     }
-    blend_resolve<K>(fp, vp, core, tail, tail_T, __uint2float_rn(static_cast<uint32_t>(px_i)),
-                     __uint2float_rn(static_cast<uint32_t>(py_i)), is_fovea ? vp.image : vp.work, px_i, py_i);
 }
 
 // The records mode's segment and merge.  The last of the tile's segments to finish merges them:
@@ -2069,12 +2388,12 @@ __device__ __forceinline__ void split_replay(const FrameParams& fp, const FrameB
 // the whole tile serially instead.
 template <int K, int RW>
 __device__ __forceinline__ void blend_split_records(const FrameParams& fp, const FrameBuffers& fb, const SplitArgs& sp,
-                                                    uint32_t g, const BlendSmem& sm, uint32_t packed, uint32_t seg0,
+                                                    uint32_t g, BlendSmem& sm, uint32_t packed, uint32_t seg0,
                                                     uint32_t S, uint32_t s, size_t stride) {
-    constexpr int NT = 256;
+    constexpr int NT = kSplitPx;
     __shared__ int s_last;
     const int tid = threadIdx.x;
-    blend_tile<K, RW, 0, 1>(fp, fb, packed, sm, SegWalk{s, S, s == 0 ? 1 : 2, sp.recs, sp.scratch + g * stride});
+    blend_tile<K, RW, 0, 2, 1>(fp, fb, packed, 0, true, sm, SegWalk{s, S, s == 0 ? 1 : 2, sp.recs, sp.scratch + g * stride});
     __threadfence();
     __syncthreads();
     if (tid == 0) s_last = atomicAdd(&sp.ctl[seg0], 1u) == S - 1u;
@@ -2084,75 +2403,58 @@ __device__ __forceinline__ void blend_split_records(const FrameParams& fp, const
     const char* base = sp.scratch + seg0 * stride;
     const int R = sp.recs;
     uint32_t most = 0;
-    for (uint32_t k = 1; k < S; ++k) most = max(most, __ldcg(reinterpret_cast<const uint32_t*>(base + k * stride) + tid));
+    for (uint32_t k = 1; k < S; ++k)
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+            most = max(most, __ldcg(reinterpret_cast<const uint32_t*>(base + k * stride) + tid + i * kBlendThreads));
     const uint32_t warp_most = __reduce_max_sync(0xffffffffu, most);
     if ((tid & 31) == 0 && warp_most > 0) atomicMax(&fb.counters[kCtrSplitRecMax], warp_most);
     if (__syncthreads_or(most > static_cast<uint32_t>(R))) {
         if (tid == 0) atomicAdd(&fb.counters[kCtrSplitFallback], 1u);
-        blend_tile<K, RW, 0, 1>(fp, fb, packed, sm, SegWalk{0u, 1u, 0, 0, nullptr});
+        blend_tile<K, RW, 0, 2, 1>(fp, fb, packed, 0, true, sm, SegWalk{0u, 1u, 0, 0, nullptr});
         return;
     }
-    // this thread's pixel (the full-resolution layout of blend_tile)
-    const int lane = tid & 31, warp = tid >> 5;
-    const int v = static_cast<int>(packed >> 24);
-    const int item = static_cast<int>(packed & (kItemLowres - 1u));
-    const ViewParams& vp = fb.views[v];
-    const uint32_t lt = fb.work_full[static_cast<size_t>(v) * fp.max_large + item];
-    const bool is_fovea = static_cast<uint32_t>(item) < fb.status[v].n_fovea_large;
-    constexpr int rw_bits = RW == 4 ? 2 : RW == 8 ? 3 : 4;
-    constexpr int rw = 1 << rw_bits, rh = 32 >> rw_bits;
-    constexpr int wx_bits = 4 - rw_bits;
-    const int px_i = static_cast<int>(lt % static_cast<uint32_t>(vp.glw)) * kTileLarge + (warp & ((1 << wx_bits) - 1)) * rw + (lane & (rw - 1));
-    const int py_i = static_cast<int>(lt / static_cast<uint32_t>(vp.glw)) * kTileLarge + (warp >> wx_bits) * rh + (lane >> rw_bits);
-    if (px_i >= vp.width || py_i >= vp.height) return;
-    Frag core[K];
-    const float* cd = reinterpret_cast<const float*>(base);
-    const uint32_t* cc = reinterpret_cast<const uint32_t*>(base + K * 4 * NT);
+    const TilePixels pp = tile_pixels<RW, 0, 2>(fp, fb, packed, 0);
+    const ViewParams& vp = fb.views[pp.v];
+    for (int px = 0; px < 2; ++px) {
+        const int py_i = px == 0 ? pp.y[0] : pp.y[1], at = tid + px * kBlendThreads;
+        if (pp.x >= vp.width || py_i >= vp.height) continue;
+        Frag core[K];
+        const float* cd = reinterpret_cast<const float*>(base);
+        const uint32_t* cc = reinterpret_cast<const uint32_t*>(base + K * 4 * NT);
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-        core[k].depth = __ldcg(cd + k * NT + tid);
-        core[k].color = __ldcg(cc + k * NT + tid);
-    }
-    float4 tail = __ldcg(reinterpret_cast<const float4*>(base + 2 * K * 4 * NT) + tid);
-    float tail_T = __ldcg(reinterpret_cast<const float*>(base + (2 * K + 4) * 4 * NT) + tid);
-    for (uint32_t k = 1; k < S; ++k) {
-        const char* b = base + k * stride;
-        const uint32_t n = __ldcg(reinterpret_cast<const uint32_t*>(b) + tid);
-        tail += __ldcg(reinterpret_cast<const float4*>(b + 4 * NT) + tid);
-        tail_T *= __ldcg(reinterpret_cast<const float*>(b + 5 * 4 * NT) + tid);
-        const float* rd = reinterpret_cast<const float*>(b + 6 * 4 * NT);
-        const float4* rp = reinterpret_cast<const float4*>(b + (6 + R) * 4 * NT);
-#pragma unroll 4
-        for (uint32_t r = 0; r < n; ++r) {
-            const float depth = __ldcg(rd + r * NT + tid);
-            float4 pm = __ldcg(rp + r * NT + tid);
-            if (depth < core[K - 1].depth) {
-                Frag f;
-                f.depth = depth;
-                f.color = pack_rgba(pm);
-#pragma unroll
-                for (int q = 0; q < K; ++q) {
-                    if (f.depth < core[q].depth) {
-                        const Frag tf = core[q];
-                        core[q] = f;
-                        f = tf;
-                    }
-                }
-                pm = unpack_rgba(f.color);
-            }
-            tail += pm;
-            tail_T *= 1.0f - pm.w;
+        for (int k = 0; k < K; ++k) {
+            core[k].depth = __ldcg(cd + k * NT + at);
+            core[k].color = __ldcg(cc + k * NT + at);
         }
+        float4 tail = __ldcg(reinterpret_cast<const float4*>(base + 2 * K * 4 * NT) + at);
+        float tail_T = __ldcg(reinterpret_cast<const float*>(base + (2 * K + 4) * 4 * NT) + at);
+        for (uint32_t k = 1; k < S; ++k) {
+            const char* b = base + k * stride;
+            const uint32_t n = __ldcg(reinterpret_cast<const uint32_t*>(b) + at);
+            tail += __ldcg(reinterpret_cast<const float4*>(b + 4 * NT) + at);
+            tail_T *= __ldcg(reinterpret_cast<const float*>(b + 5 * 4 * NT) + at);
+            const float* rd = reinterpret_cast<const float*>(b + 6 * 4 * NT);
+            const float4* rp = reinterpret_cast<const float4*>(b + (6 + R) * 4 * NT);
+#pragma unroll 4
+            for (uint32_t r = 0; r < n; ++r) {
+                const float depth = __ldcg(rd + r * NT + at);
+                float4 pm = __ldcg(rp + r * NT + at);
+                if (depth < core[K - 1].depth) pm = unpack_rgba(core_insert<K>(core, depth, pm));
+                tail += pm;
+                tail_T *= 1.0f - pm.w;
+            }
+        }
+        blend_resolve<K>(fp, vp, core, tail, tail_T, __uint2float_rn(static_cast<uint32_t>(pp.x)),
+                         __uint2float_rn(static_cast<uint32_t>(py_i)), pp.is_fovea ? vp.image : vp.work, pp.x, py_i);
     }
-    blend_resolve<K>(fp, vp, core, tail, tail_T, __uint2float_rn(static_cast<uint32_t>(px_i)),
-                     __uint2float_rn(static_cast<uint32_t>(py_i)), is_fovea ? vp.image : vp.work, px_i, py_i);
 }
 
 // One segment of a split full-resolution tile (split list entry g): the exact split's log and
 // replay (EXACT), or the records mode's segment and merge.
 template <int K, int RW, bool EXACT>
 __device__ __forceinline__ void blend_split_segment(const FrameParams& fp, const FrameBuffers& fb, const SplitArgs& sp,
-                                                    uint32_t g, const BlendSmem& sm) {
+                                                    uint32_t g, BlendSmem& sm) {
     __shared__ int s_last;
     const int tid = threadIdx.x;
     const uint2 e = sp.list[g];
@@ -2160,12 +2462,12 @@ __device__ __forceinline__ void blend_split_segment(const FrameParams& fp, const
     const uint32_t packed = e.x, seg0 = e.y & 0x0fffffffu, S = e.y >> 28, s = g - seg0;
     const size_t stride = static_cast<size_t>(sp.stride);
     if constexpr (EXACT) {
-        const int v = static_cast<int>(packed >> 24);
-        const uint32_t lt = fb.work_full[static_cast<size_t>(v) * fp.max_large + (packed & (kItemLowres - 1u))];
+        const int v = item_view(packed);
+        const uint32_t lt = fb.work_full[static_cast<size_t>(v) * fp.max_large + item_index(packed)];
         const uint2 r = fb.ranges[static_cast<size_t>(v) * fp.max_large + lt];
         const uint32_t len = r.y > r.x ? r.y - r.x : 0u;
-        const uint32_t log_stride = (len + S - 1u) / S;  // steps a warp of one segment can take
-        blend_tile<K, RW, 0, 3>(fp, fb, packed, sm,
+        const uint32_t log_stride = (len + S - 1u) / S;  // steps a group of one segment can take
+        blend_tile<K, RW, 0, 2, 3>(fp, fb, packed, 0, true, sm,
                                 SegWalk{s, S, 3, static_cast<int>(log_stride), sp.pool + 256ull * sp.seg_unit[g]});
         __threadfence();
         __syncthreads();
@@ -2184,73 +2486,57 @@ __device__ __forceinline__ void blend_split_segment(const FrameParams& fp, const
 // the other tiles (launched after it as its programmatic dependent) start at once, so that
 // those blocks take the SMs as this kernel's blocks run out of segments.
 template <int K, int RW, bool EXACT>
-__global__ void __launch_bounds__(256, blend_min_blocks(K)) blend_split_kernel(FrameParams fp, FrameBuffers fb,
-                                                                              SplitArgs sp) {
+__global__ void __launch_bounds__(kBlendThreads, blend_blocks(K)) blend_split_kernel(FrameParams fp, FrameBuffers fb,
+                                                                                    SplitArgs sp) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    constexpr int NT = 256;
-    constexpr int NW = NT / 32;
-    __shared__ float4 s_p1[NT], s_p2[NT], s_p4[NT], s_rgba[NT];
-    __shared__ uint32_t s_mask[NT];
-    __shared__ uint8_t s_list[NW][NT];
-    __shared__ int s_item;
-    const BlendSmem sm{s_p1, s_p2, s_p4, s_rgba, s_mask, s_list};
+    __shared__ BlendSmem sm;
+    blend_smem_init(sm);
     const uint32_t n_seg = min(fb.counters[kCtrSplitSegs], static_cast<uint32_t>(sp.cap));
     for (;;) {
-        if (threadIdx.x == 0) s_item = static_cast<int>(atomicAdd(&fb.counters[kCtrSplitNext], 1u));
+        if (threadIdx.x == 0) sm.item = static_cast<int>(atomicAdd(&fb.counters[kCtrSplitNext], 1u));
         __syncthreads();
-        const uint32_t g = static_cast<uint32_t>(s_item);
+        const uint32_t g = static_cast<uint32_t>(sm.item);
         __syncthreads();
         if (g >= n_seg) break;
         blend_split_segment<K, RW, EXACT>(fp, fb, sp, g, sm);
     }
 }
 
-// One persistent kernel blends every tile of every view.  The work list holds the full-resolution
-// tiles, then the periphery tiles, then the quarter tiles, each class heaviest first; blocks take
-// items class by class, each class with its own compiled tile code.
-// SPLIT: launched after blend_split_kernel as its programmatic dependent, with the status whose
-// full-resolution counts leave out the split tiles (which the work order left out of its list).
+// One persistent kernel blends every tile of every view, block item by block item of the work
+// list.
+// SPLIT: launched after blend_split_kernel as its programmatic dependent (the work order left the
+// split tiles out of the list).
 template <int K, int RW, bool SPLIT>
-__global__ void __launch_bounds__(256, blend_min_blocks(K)) blend_kernel(FrameParams fp, FrameBuffers fb) {
-    constexpr int NT = 256;
-    constexpr int NW = NT / 32;
-    __shared__ float4 s_p1[NT], s_p2[NT], s_p4[NT], s_rgba[NT];
-    __shared__ uint32_t s_mask[NT];
-    __shared__ uint8_t s_list[NW][NT];
-    __shared__ int s_item;
-    const BlendSmem sm{s_p1, s_p2, s_p4, s_rgba, s_mask, s_list};
-    const int tid = threadIdx.x;
-    int n_full = 0, n_half = 0, n_quarter = 0;
-    for (int v = 0; v < fp.n_views; ++v) {
-        const FrameStatus& st = fb.status[v];
-        n_full += static_cast<int>(st.n_fovea_large + st.n_blended_large);
-        n_half += static_cast<int>(st.n_periphery_large);
-        n_quarter += static_cast<int>(st.n_quarter_large);
+__global__ void __launch_bounds__(kBlendThreads, blend_blocks(K)) blend_kernel(FrameParams fp, FrameBuffers fb) {
+    __shared__ BlendSmem sm;
+    // the blocks that the work order wants resident (the first ones are spread over all SMs)
+    if (blockIdx.x >= fb.counters[kCtrBlocks]) {
+        if constexpr (SPLIT) asm volatile("griddepcontrol.wait;" ::: "memory");
+        return;
     }
-    const uint32_t* order = fb.work_order[0];
-    for (;;) {  // full-resolution tiles (listed first)
-        if (tid == 0) s_item = static_cast<int>(atomicAdd(&fb.counters[0], 1u));
+    blend_smem_init(sm);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t n_items = fb.counters[kCtrItems], n_low = fb.counters[kCtrLow], n_quarter = fb.counters[kCtrQuarter];
+    const uint32_t* runs = fb.work_order[1];
+    for (;;) {
+        if (tid == 0) sm.item = static_cast<int>(atomicAdd(&fb.counters[kCtrNext], 1u));
         __syncthreads();
-        const int g = s_item;
+        const uint32_t g = static_cast<uint32_t>(sm.item);
         __syncthreads();
-        if (g >= n_full) break;
-        blend_tile<K, RW, 0>(fp, fb, order[g], sm);
-    }
-    for (;;) {  // periphery tiles
-        if (tid == 0) s_item = static_cast<int>(atomicAdd(&fb.counters[1], 1u));
-        __syncthreads();
-        const int g = s_item;
-        __syncthreads();
-        if (g >= n_half) break;
-        blend_tile<K, RW, 1>(fp, fb, order[n_full + g], sm);
-    }
-    for (;;) {  // ring-mode quarter tiles
-        if (tid == 0) s_item = static_cast<int>(atomicAdd(&fb.counters[2], 1u));
-        __syncthreads();
-        const int g = s_item;
-        __syncthreads();
-        if (g >= n_quarter) break;
-        blend_tile<K, RW, 2>(fp, fb, order[n_full + n_half + g], sm);
+        if (g >= n_items) break;
+        const uint32_t item = fb.work_order[0][g], kind = item >> kItemKindShift;
+        if (kind == kItemFull) {
+            blend_tile<K, RW, 0, 2>(fp, fb, item, 0, true, sm);
+        } else if (kind == kItemHalf || kind == kItemHalf + 1u) {
+            blend_tile<K, RW, 0, 1>(fp, fb, item, static_cast<int>(kind - kItemHalf), true, sm);
+        } else if (kind == kItemLow) {
+            const uint32_t i = (item & kItemNumberMask) * kLowTiles + warp;
+            if (i < n_low) blend_tile<K, RW, 1, 2>(fp, fb, runs[i], 0, true, sm);
+        } else {
+            const uint32_t i0 = (item & kItemNumberMask) * kQuarterTiles + 4 * warp, i = i0 + (lane >> 3);
+            if (i0 < n_quarter)
+                blend_tile<K, RW, 2, 2>(fp, fb, runs[n_low + (i < n_quarter ? i : i0)], 0, i < n_quarter, sm);
+        }
     }
     // this grid completes only after the split kernel's has
     if constexpr (SPLIT) asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -2260,32 +2546,30 @@ template <int K, int RW>
 int launch_blend_kr(const FrameParams& fp, const FrameBuffers& fb, const SplitArgs& sp, int n_sms, cudaStream_t s,
                     cudaEvent_t mid) {
     static int occ = -1, occ_split = -1;  // per instantiation, queried once
-    if (occ < 0) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, blend_kernel<K, RW, false>, 256, 0);
+    if (occ < 0) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, blend_kernel<K, RW, false>, kBlendThreads, 0);
     int per_sm = occ > 0 ? occ : 1;
     if (fp.blend_blocks > 0 && fp.blend_blocks < per_sm) per_sm = fp.blend_blocks;
     if (!(sp.share > 0.0f) || sp.of == nullptr) {
-        blend_kernel<K, RW, false><<<n_sms * per_sm, 256, 0, s>>>(fp, fb);
+        blend_kernel<K, RW, false><<<n_sms * per_sm, kBlendThreads, 0, s>>>(fp, fb);
         if (mid) cudaEventRecord(mid, s);
         return 1;
     }
-    if (occ_split < 0) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_split, blend_split_kernel<K, RW, false>, 256, 0);
+    if (occ_split < 0) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_split, blend_split_kernel<K, RW, false>, kBlendThreads, 0);
     int per_sm_split = occ_split > 0 ? occ_split : 1;
     if (fp.blend_blocks > 0 && fp.blend_blocks < per_sm_split) per_sm_split = fp.blend_blocks;
-    if (sp.exact) blend_split_kernel<K, RW, true><<<n_sms * per_sm_split, 256, 0, s>>>(fp, fb, sp);
-    else blend_split_kernel<K, RW, false><<<n_sms * per_sm_split, 256, 0, s>>>(fp, fb, sp);
+    if (sp.exact) blend_split_kernel<K, RW, true><<<n_sms * per_sm_split, kBlendThreads, 0, s>>>(fp, fb, sp);
+    else blend_split_kernel<K, RW, false><<<n_sms * per_sm_split, kBlendThreads, 0, s>>>(fp, fb, sp);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(n_sms * per_sm);
-    cfg.blockDim = dim3(256);
+    cfg.blockDim = dim3(kBlendThreads);
     cfg.dynamicSmemBytes = 0;
     cfg.stream = s;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    FrameBuffers rest = fb;  // the other tiles: the status without the split tiles
-    rest.status = sp.status;
-    cudaLaunchKernelEx(&cfg, blend_kernel<K, RW, true>, fp, rest);
+    cudaLaunchKernelEx(&cfg, blend_kernel<K, RW, true>, fp, fb);
     if (mid) cudaEventRecord(mid, s);
     return 2;
 }

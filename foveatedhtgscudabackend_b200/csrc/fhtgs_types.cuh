@@ -85,8 +85,8 @@ struct FrameParams {
     int max_tiles;         // max small-tile ids over views (stride of per-tile arrays)
     int max_large;         // max large tiles over views
     int n_blocks_prim;     // preprocess/create blocks per view
-    int blend_rw;          // blend: pixels per warp row (4, 8 or 16; 32 / blend_rw rows)
-    int blend_blocks;      // persistent blend blocks per SM (0: as many as fit)
+    int blend_rw;          // blend: rectangle of a 16-sample group (8: 4 x 4, 16: 8 x 2, 4: 2 x 8)
+    int blend_blocks;      // most persistent blend blocks per SM (0: as many as fit)
     int sort_key_bits;     // three-kernel sort: > 0 = only key bits below this decide the order
                            // (higher bits are carried along, as cub's end_bit); 0 = all bits of
                            // the sort's 8-bit passes (the renderer's keys have no higher bits)
@@ -151,20 +151,20 @@ struct FrameBuffers {
     uint32_t* work_low;       // [V][max_large] periphery large tiles, then quarter tiles
     uint32_t* work_masked;    // [V][max_large] masked large tiles
     uint32_t* counters;       // [kCounterWords]: work counters, then the work-order buckets
-    uint32_t* work_order[2];  // [0]: [V*max_large] packed blend items, heaviest first; [1] unused
+    uint32_t* work_order[2];  // [0]: [2*V*max_large] the blend's block items, longest first;
+                              // [1]: [V*max_large] the tiles of its periphery and quarter items
     // Onesweep sort state (null: the three-kernel sort, which needs sort_hist/sort_digit_tot):
     uint32_t* sort_ghist;     // [V][kSortMaxPasses][256] digit counts of every pass (create fills)
     uint32_t* sort_look;      // [V][kSortMaxPasses][sort_tiles][256] look-back words
     uint32_t* sort_ticket;    // [V][kSortMaxPasses] tiles handed out so far
 };
 
-// Work ordering: tiles are bucketed by class and by list length in quarter octaves and
-// blended in descending bucket order: full-resolution tiles, then periphery, then quarter
-// tiles, the longest lists of each class first (longest-processing-time scheduling).
+// Work ordering: tiles are bucketed by class and by estimated duration in quarter octaves.
 constexpr int kCostBuckets = 130;                     // per tile class
-constexpr int kOrderBuckets = 3 * kCostBuckets;       // full-resolution, periphery, quarter
-// counters[0..2]: next full-resolution / periphery / quarter item of the blend; then the split
-// blend's words; the work-order histogram and cursors follow from kCtrHist.
+constexpr int kOrderBuckets = 3 * kCostBuckets;       // quarter, periphery, full-resolution
+// counters: the blend's next block item; the split blend's words; the work order's totals
+// (block items, periphery tiles, quarter tiles, costs), histogram and cursors.
+constexpr int kCtrNext = 0;
 constexpr int kCtrSplitNext = 3;      // next split segment of the blend
 constexpr int kCtrSplitSegs = 4;      // segments reserved by the work order
 constexpr int kCtrSplitTiles = 5;     // tiles split
@@ -172,14 +172,18 @@ constexpr int kCtrSplitFallback = 6;  // split tiles blended whole after a recor
 constexpr int kCtrSplitRecMax = 7;    // most records a pixel of a later segment produced
 constexpr int kCtrSplitPool = 8;      // exact mode: 256-byte units of the fragment log reserved
                                       // (64-bit: words 8 and 9)
-constexpr int kCtrSplitView = 16;     // [256] tiles split per view
-constexpr int kCtrHist = kCtrSplitView + 256;
+constexpr int kCtrItems = 10, kCtrLow = 11, kCtrQuarter = 12;
+// the items' total and longest estimated cost (floats) and the blend blocks to use
+constexpr int kCtrCost = 13, kCtrLongest = 14, kCtrBlocks = 15;
+constexpr int kCtrHist = 16;
 constexpr int kCounterWords = kCtrHist + 2 * kOrderBuckets;  // counters, histogram, cursors
 constexpr int kSplitMaxSegments = 8;
 
-// Persistent blend blocks per SM the register allocation has to allow: the K-buffer (2 K
-// registers) dominates for large K.
-__host__ __device__ constexpr int blend_min_blocks(int K) { return K >= 32 ? 2 : K >= 16 ? 3 : 4; }
+// Persistent blend blocks (of 128 threads) per SM the register allocation has to allow: the two
+// K-buffers of a thread (4 K registers) dominate for large K.
+__host__ __device__ constexpr int blend_blocks(int K) { return K >= 32 ? 2 : K >= 16 ? 3 : 5; }
+// The block count the split blend's segment share refers to (fhtgs_context_set_blend_split).
+__host__ __device__ constexpr int split_share_blocks(int K) { return K >= 32 ? 2 : K >= 16 ? 3 : 4; }
 
 // Split blend (a tolerance mode, off by default; its own kernel argument so that the other
 // kernels' parameters keep their layout): a full-resolution tile whose list is longer than
@@ -195,10 +199,6 @@ struct SplitArgs {
     uint2* list;           // [cap] per segment: packed item, first segment | S << 28 (~0: unused)
     uint32_t* ctl;         // [cap] per first segment: segments finished
     char* scratch;         // [cap][stride] per-pixel state and records
-    // [V] the status the blend of the other tiles reads: the view's, with the split tiles taken
-    // out of n_fovea_large + n_blended_large (that kernel reads only this sum, and n_fovea_large,
-    // which is kept; n_blended_large is adjusted modulo 2^32)
-    FrameStatus* status;
     // Exact mode (bit-identical images): every segment logs, per pixel and in list order, the
     // alpha and depth of each Gaussian its warp evaluates; the last segment of a tile replays the
     // whole log with the walk's own K-buffer and tail steps.
@@ -208,11 +208,12 @@ struct SplitArgs {
     uint32_t* seg_unit;    // [cap] first unit of each segment's log
 };
 
-// Exact split: a segment's log, for a segment of at most `stride` list entries (each warp walks
-// at most that many steps): n_steps[8] u32 | rgba[8][stride] float4 (each step's Gaussian colour
-// and opacity) | frag[8][stride][32] float2 (alpha, or -1 where the pair is no fragment; depth).
+// Exact split: a segment's log, for a segment of at most `stride` list entries (each group of 16
+// pixels walks at most that many steps): n_steps[16] u32 | rgba[16][stride] float4 (each step's
+// Gaussian colour and opacity) | frag[16][stride][16] float2 (alpha, or -1 where the pair is no
+// fragment; depth).
 __host__ __device__ inline uint32_t split_log_pos_unit() { return 1u; }
-__host__ __device__ inline uint32_t split_log_frag_unit(uint32_t stride) { return 1u + (stride + 1u) / 2u; }
+__host__ __device__ inline uint32_t split_log_frag_unit(uint32_t stride) { return 1u + stride; }
 __host__ __device__ inline uint32_t split_log_units(uint32_t stride) { return split_log_frag_unit(stride) + 8u * stride; }
 
 // Split blend scratch of one segment (256 pixels; arrays pixel-fastest):
@@ -251,7 +252,7 @@ constexpr int kSortThreads = 256;
 constexpr int kSortItems = 16;        // default keys per thread per sort tile
 constexpr int kSortTile = kSortThreads * kSortItems;  // 4096 (default tile)
 constexpr int kSortItemsMin = 8;      // smallest tile the autotuner may choose (2048 keys)
-// Blend warp rectangles the autotuner may choose: pixels per warp row.
+// Blend group rectangles the autotuner may choose (FrameParams.blend_rw).
 constexpr int kBlendRowChoices[3] = {8, 16, 4};
 constexpr int kSortRadixBits = 8;
 constexpr int kSortBins = 1 << kSortRadixBits;

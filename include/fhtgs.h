@@ -305,8 +305,10 @@ fhtgs_status fhtgs_sort_instances_noalloc(const void* keys_in, const uint32_t* v
  *
  * Tuning knobs of a context; every choice renders identical images (they change which pairs
  * the blend culls as hopeless and how the sort is tiled, never a pixel's arithmetic):
- *   blend_warp_width     pixels per warp row in the blend: 8 (8x4 pixels), 16 (16x2) or 4 (4x8)
- *   blend_blocks_per_sm  persistent blend blocks per SM; 0 = as many as fit
+ *   blend_warp_width     rectangle of the blend's 16-pixel culling groups: 8 (4x4 pixels), 16
+ *                        (8x2) or 4 (2x8)
+ *   blend_blocks_per_sm  most persistent blend blocks per SM; 0 = as many as fit (a frame that
+ *                        ends with a few long tiles uses fewer by itself)
  *   sort_items           keys per thread of a radix-sort tile: 8, 12 or 16 (tile = 256 x items) */
 typedef struct fhtgs_tuning {
     int32_t blend_warp_width;
