@@ -1833,7 +1833,7 @@ __device__ __forceinline__ float sqrt_approx(float x) {
 // its x extent over a row of groups gives that row's bits at once (one test per row of groups
 // instead of one per group).  Ellipses that are not clearly ellipses, or out of the range of the
 // approximate arithmetic, are tested by their bounding box; unbounded ones reach every group, and
-// so do Gaussians so small (F0 = -rc |d|^2 at the mean) that the blend's 1 / |d|^2 may overflow:
+// so do Gaussians so small (rc |d|^2 at the mean) that the blend's 1 / |d|^2 may overflow:
 // 0 x inf makes their alpha 1 at any pixel of their tiles.
 // Rows row0 .. row0 + ROWS_USED - 1 of groups are tested (a half item's).
 // `zmin` receives a depth that no fragment of the core (alpha >= 1/20) undercuts: the depth is
@@ -1852,8 +1852,7 @@ __device__ __forceinline__ uint32_t reached_groups(const float4 P1, const float4
     if (!(P4.w > 0.0f) || !(rc > 0.0f) || !(P4.w * P4.w - rc * nn > 0.0f)) return valid;
     Conic q;
     const bool ell = cutoff_conic(P1, P2, P4, opacity, q) && q.det > 1e-3f * (4.0f * q.A * q.C) && q.A < 1e30f &&
-                     q.C < 1e30f && q.det < 1e30f && q.A > 1e-30f && q.C > 1e-30f && q.det > 1e-30f;
-    if (!(q.F0 < -1e-28f)) return valid;
+                     q.C < 1e30f && q.det < 1e30f && q.A > 1e-30f && q.C > 1e-30f && q.det > 1e-30f && q.F0 < -1e-28f;
     uint32_t m = 0u;
     if (ell) {
         const float idet = rcp_approx(q.det), i2a = 0.5f * rcp_approx(q.A), i2c = 0.5f * rcp_approx(q.C);
@@ -1887,9 +1886,11 @@ __device__ __forceinline__ uint32_t reached_groups(const float4 P1, const float4
             zmin = P4.w - (1.25f * sqrt_approx(fmaxf(rho2, 0.0f)) + 0.5f) * sqrt_approx(nn) - 1e-4f * P4.w;
         return m & valid;
     }
+    const float ix = P1.w / P4.w, iy = P2.w / P4.w;
+    const float3 c0 = cross(xyz(P1) - ix * n4, xyz(P2) - iy * n4);  // the direction vector d at the mean
     float4 box;
     bool never;
-    if (!cutoff_box(P1, P2, P4, opacity, box, never)) return valid;
+    if (!(rc * dot(c0, c0) > 1e-28f) || !cutoff_box(P1, P2, P4, opacity, box, never)) return valid;
     if (never) return 0u;
     for (int g = 0; g < G::COLS * G::ROWS; ++g) {
         const float ax0 = ox + static_cast<float>((g % G::COLS) * G::GW) * fS, ax1 = ax0 + static_cast<float>(G::GW - 1) * fS;
