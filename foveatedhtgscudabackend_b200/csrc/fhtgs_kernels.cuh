@@ -1314,11 +1314,11 @@ int launch_ranges(const FrameParams& fp, const FrameBuffers& fb, int n_sms, cuda
 //   full    a full-resolution tile, two pixels a thread
 //   half    the upper or lower half of a full-resolution tile, one pixel a thread: the tiles
 //           whose walk alone would outlast the frame's mean work per block
-//   low     four periphery tiles, one per warp
+//   low     four periphery tiles, or halves of them, one per warp
 //   quarter sixteen ring-mode quarter tiles, four per warp
 // An item word is kind << 29 | view << 21 | index into the view's work_full list, or kind << 29 |
-// item number for the last two, whose tiles lie in work_order[1] (view << 21 | index into
-// work_low), longest first: the periphery tiles of all views, then the quarter tiles.
+// item number for the last two, whose tiles lie in work_order[1] (the same word, with the index
+// into work_low), longest first: the periphery tiles of all views, then the quarter tiles.
 // ------------------------------------------------------------------------------------------
 constexpr uint32_t kItemFull = 0u, kItemHalf = 1u /* and 2 */, kItemLow = 3u, kItemQuarter = 4u;
 constexpr int kItemKindShift = 29, kItemViewShift = 21;
@@ -1326,13 +1326,14 @@ constexpr uint32_t kItemIndexMask = (1u << kItemViewShift) - 1u;
 constexpr uint32_t kItemNumberMask = (1u << kItemKindShift) - 1u;
 __device__ __forceinline__ int item_view(uint32_t packed) { return static_cast<int>((packed >> kItemViewShift) & 255u); }
 __device__ __forceinline__ uint32_t item_index(uint32_t packed) { return packed & kItemIndexMask; }
-// Tiles of a low / quarter item.
+// Tiles (or halves) of a low / quarter item.
 constexpr uint32_t kLowTiles = 4, kQuarterTiles = 16;
 
 // Estimated duration of an item in list entries of a full item: per entry of its (longest) list,
-// plus the item's fixed cost.  Measured on the stereo frames: 148 ns per entry of a full item and
-// 115 of a half item at four blocks per SM, 230 of a periphery item, about 5 us fixed.
-constexpr float kCostHalf = 0.75f, kCostLow = 1.6f, kCostQuarter = 2.5f, kCostItem = 32.0f;
+// plus the item's fixed cost.  Measured at five blocks per SM: 168 ns per entry of a full item and
+// 90 of a half item (stereo frame), 144 and 208 of a full and a periphery item (6M Gaussians,
+// rings), about 5 us fixed.
+constexpr float kCostHalf = 0.6f, kCostLow = 1.6f, kCostQuarter = 2.5f, kCostItem = 32.0f;
 // A full-resolution tile becomes two half items when its list is longer than this share of the
 // frame's instances per SM: its walk would then outlast the frame at five blocks per SM.
 constexpr float kHalfShare = 0.16f;
@@ -1386,8 +1387,12 @@ __device__ __forceinline__ int item_tile(const FrameParams& fp, const FrameBuffe
 
 // Estimated duration of a tile's item (class 2: full or half), see kCostHalf.
 __device__ __forceinline__ float item_cost(int cls, uint32_t len, bool halves) {
-    const float c = cls == 2 ? (halves ? kCostHalf : 1.0f) : cls == 1 ? kCostLow : kCostQuarter;
-    return c * static_cast<float>(len) + kCostItem;
+    const float c = cls == 2 ? 1.0f : cls == 1 ? kCostLow : kCostQuarter;
+    return c * (halves ? kCostHalf : 1.0f) * static_cast<float>(len) + kCostItem;
+}
+// Does the tile become two half items (half_threshold)?
+__device__ __forceinline__ bool blend_halves(int cls, uint32_t len, uint32_t half_len) {
+    return cls == 2 ? len > half_len : cls == 1 && kCostLow * static_cast<float>(len) > static_cast<float>(half_len);
 }
 // Its bucket: class above duration bucket.
 __device__ __forceinline__ int item_bucket(int cls, float cost) { return cls * kCostBuckets + cost_bucket(cost); }
@@ -1483,10 +1488,10 @@ __global__ void __launch_bounds__(256) order_hist_kernel(FrameParams fp, FrameBu
             sp.of[static_cast<size_t>(v) * fp.max_large + j] = tag;
             if (tag != ~0u) continue;
         }
-        const bool halves = cls == 2 && len > half_len;
+        const bool halves = blend_halves(cls, len, half_len);
         const float cost = item_cost(cls, len, halves);
         longest = fmaxf(longest, cost);
-        cost_sum += cost * (cls == 2 ? (halves ? 2.0f : 1.0f) : 1.0f / (cls == 1 ? kLowTiles : kQuarterTiles));
+        cost_sum += cost * (halves ? 2.0f : 1.0f) / static_cast<float>(cls == 2 ? 1u : cls == 1 ? kLowTiles : kQuarterTiles);
         atomicAdd(&hist[item_bucket(cls, cost)], halves ? 2u : 1u);
     }
 #pragma unroll
@@ -1575,7 +1580,7 @@ __global__ void __launch_bounds__(256) order_scatter_kernel(FrameParams fp, Fram
             item_of(g, pre, fp.n_views, v, j);
             uint32_t len;
             cls = item_tile(fp, fb, v, j, len, packed);
-            halves = cls == 2 && len > half_len;
+            halves = blend_halves(cls, len, half_len);
             b = item_bucket(cls, item_cost(cls, len, halves));
             if (sp.of != nullptr && sp.share > 0.0f && cls == 2) {
                 const uint32_t tag = sp.of[static_cast<size_t>(v) * fp.max_large + j];
@@ -1603,11 +1608,14 @@ __global__ void __launch_bounds__(256) order_scatter_kernel(FrameParams fp, Fram
                     out[place] = (kItemFull << kItemKindShift) | packed;
                 }
             } else {
-                runs[at - n_full] = packed;
+                const uint32_t kind = halves ? kItemHalf : kItemFull;
+                runs[at - n_full] = (kind << kItemKindShift) | packed;
+                if (halves) runs[at - n_full + 1] = ((kind + 1u) << kItemKindShift) | packed;
                 const uint32_t per = cls == 1 ? kLowTiles : kQuarterTiles, k = at - n_full - (cls == 1 ? 0u : n_low);
-                if (k % per == 0)  // the first tile of an item
-                    out[k / per + at_least(2, d) + (cls == 1 ? quarter_items(d + 1) : low_items(d))] =
-                        ((cls == 1 ? kItemLow : kItemQuarter) << kItemKindShift) | (k / per);
+                const uint32_t first = (k + per - 1) / per * per;
+                if (first < k + (halves ? 2u : 1u))  // the first tile (or half) of an item
+                    out[first / per + at_least(2, d) + (cls == 1 ? quarter_items(d + 1) : low_items(d))] =
+                        ((cls == 1 ? kItemLow : kItemQuarter) << kItemKindShift) | (first / per);
             }
         }
         __syncthreads();  // the counts are cleared for the next round
@@ -1642,10 +1650,13 @@ int launch_order(const FrameParams& fp, const FrameBuffers& fb, const SplitArgs&
 //     evaluate it instead of half;
 //   - one x interval per row of groups instead of a test per rectangle; selections instead of
 //     branches in the K-buffer insertion;
-//   - half items and fewer blocks per SM for frames that end with a few long tiles (work order).
+//   - half items (one pixel a lane, two list entries a step: 1.07 times the work of the whole
+//     tile in about half its time) and fewer blocks per SM for frames that end with a few long
+//     tiles (work order).
 // Blend of the stereo frame (1M Gaussians, 2 x 2064x2208, K = 8) 4.87 -> 3.30 ms, of 12 views of
-// 1920x1080 10.65 -> 6.65 ms, of the plain 1280x720 view (100k, K = 4) 0.73 -> 0.20 ms, of a
-// 2 x 1032x1104 frame of the 1M scene 5.3 -> 1.84 ms, K = 32 at 1280x720 0.72 -> 0.56 ms.
+// 1920x1080 10.65 -> 6.7 ms, of the plain 1280x720 view (100k, K = 4) 0.73 -> 0.18 ms, of a
+// 2 x 1032x1104 frame of the 1M scene 5.3 -> 1.7 ms, of 6M with rings 27.8 -> 16.2 ms, K = 32 at
+// 1280x720 0.72 -> 0.54 ms.
 // ------------------------------------------------------------------------------------------
 struct Frag {
     float depth;
@@ -1907,7 +1918,8 @@ __device__ __forceinline__ uint32_t reached_groups(const float4 P1, const float4
 constexpr int kBlendThreads = 128;
 constexpr int kBlendWarps = kBlendThreads / 32;
 constexpr int kBlendGroups = 4 * kBlendWarps;
-constexpr int kBlendSlots = 2 * kBlendThreads;  // staged Gaussians: two per thread
+constexpr int kBlendPerThread = 3;  // Gaussians a thread stages (2: 12 views 6.63 instead of 6.59 ms)
+constexpr int kBlendSlots = kBlendPerThread * kBlendThreads;
 constexpr int kBlendDummy = kBlendSlots;
 struct BlendSmem {
     float4 p1[kBlendSlots + 1], p2[kBlendSlots + 1], p4[kBlendSlots + 1], rgba[kBlendSlots + 1];
@@ -2033,7 +2045,7 @@ __device__ __forceinline__ TilePixels tile_pixels(const FrameParams& fp, const F
     constexpr int LPG = 16 / PX, GPW = 32 / LPG;  // lanes per group, groups per warp
     TilePixels tp;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k = lane % LPG;
-    const int group = CLS == 0 ? half * kBlendWarps * GPW + GPW * warp + lane / LPG : CLS == 1 ? lane / LPG : 0;
+    const int group = CLS == 0 ? (half * kBlendWarps + warp) * GPW + lane / LPG : CLS == 1 ? half * GPW + lane / LPG : 0;
     tp.v = item_view(packed);
     const uint32_t item = item_index(packed);
     const ViewParams& vp = fb.views[tp.v];
@@ -2048,8 +2060,8 @@ __device__ __forceinline__ TilePixels tile_pixels(const FrameParams& fp, const F
 }
 
 // Blends one tile, or half of one (PX 1: `half`), with a team of threads: the block (CLS 0), a
-// warp (CLS 1) or 8 lanes (CLS 2; `live` false: no tile for this group).  The team stages its tile's list two
-// Gaussians a thread at a time; every thread culls its two against the tile's sample groups, each
+// warp (CLS 1) or 8 lanes (CLS 2; `live` false: no tile for this group).  The team stages its tile's list
+// kBlendPerThread Gaussians a thread at a time; every thread culls its own against the tile's sample groups, each
 // group's survivors become its list, and the warp walks its groups' lists side by side, in list
 // order.  Which pairs are culled (pairs that cannot pass the alpha test) never changes a
 // pixel's arithmetic.
@@ -2058,11 +2070,12 @@ __device__ __forceinline__ void blend_tile(const FrameParams& fp, const FrameBuf
                                            BlendSmem& sm, const SegWalk sw = SegWalk{0u, 1u, 0, 0, nullptr}) {
     using G = GroupShape<RW, CLS>;
     constexpr uint32_t TEAM = CLS == 0 ? kBlendThreads : CLS == 1 ? 32 : 8;
-    constexpr uint32_t BATCH = 2 * TEAM;
+    constexpr uint32_t BATCH = kBlendPerThread * TEAM;
     constexpr bool log_mode = SEG == 3;  // the exact split's segment: log the fragments only
     constexpr int NT = kSplitPx;
     constexpr int LPG = 16 / PX, GPW = 32 / LPG;  // lanes per group, groups per warp
-    static_assert(PX == 2 || (CLS == 0 && SEG == 0), "half items are full-resolution");
+    constexpr uint32_t EPS = 2 / PX;              // list entries a step evaluates
+    static_assert(PX == 2 || (CLS != 2 && SEG == 0), "no halves of quarter tiles and of split segments");
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, grp = lane / LPG;
     const uint32_t team_tid = CLS == 0 ? tid : CLS == 1 ? lane : lane & 7;
     const uint32_t team_base = CLS == 0 ? 0u : CLS == 1 ? warp * BATCH : (warp * 4 + grp) * BATCH;
@@ -2074,12 +2087,13 @@ __device__ __forceinline__ void blend_tile(const FrameParams& fp, const FrameBuf
 #pragma unroll
     for (int i = 0; i < PX; ++i) pixel_y[i] = __uint2float_rn(static_cast<uint32_t>(pp.y[i]));
     const f32x2 npixel_y = pair(-pixel_y[0], -pixel_y[PX - 1]);
-    constexpr int ROWS_USED = CLS == 0 ? G::ROWS * PX / 2 : G::ROWS;
-    const int row0 = half * ROWS_USED;
-    uint32_t valid = 0u;  // this item's groups with a pixel inside the image
+    // this item's groups, those with a pixel inside the image, and the rows they lie in
+    constexpr int NG = CLS == 2 ? 1 : G::COLS * G::ROWS * PX / 2, ROWS_USED = NG >= G::COLS ? NG / G::COLS : 1;
+    const int row0 = half * NG / G::COLS;
+    uint32_t valid = 0u;
 #pragma unroll
-    for (int i = 0; i < G::COLS * ROWS_USED; ++i) {
-        const int g = row0 * G::COLS + i;
+    for (int i = 0; i < NG; ++i) {
+        const int g = half * NG + i;
         if (pp.ox + (g % G::COLS) * G::GW * G::S < vp.width && pp.oy + (g / G::COLS) * G::GH * G::S < vp.height) valid |= 1u << g;
     }
     uint2 range = live ? fb.ranges[static_cast<size_t>(pp.v) * fp.max_large + pp.lt] : make_uint2(0u, 0u);
@@ -2108,9 +2122,9 @@ __device__ __forceinline__ void blend_tile(const FrameParams& fp, const FrameBuf
     for (uint32_t start = range.x; CLS == 2 ? __any_sync(0xffffffffu, start < range.y) : start < range.y; start += BATCH) {
         const uint32_t n_batch = start < range.y ? min(BATCH, range.y - start) : 0u;
         if (CLS == 0) __syncthreads(); else __syncwarp();
-        uint32_t mask[2];
+        uint32_t mask[kBlendPerThread];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
+        for (int h = 0; h < kBlendPerThread; ++h) {
             const uint32_t i = h * TEAM + team_tid, slot = team_base + i;
             mask[h] = 0u;
             const uint32_t p = i < n_batch ? vals[start + i] : kNoPrimitive;
@@ -2134,14 +2148,14 @@ __device__ __forceinline__ void blend_tile(const FrameParams& fp, const FrameBuf
             uint32_t n[GPW] = {};
             for (uint32_t c0 = 0; c0 < n_batch; c0 += 32) {
                 const uint32_t slot = team_base + c0 + lane;
-                const uint32_t mk = sm.mask[slot] >> (CLS == 0 ? (half * kBlendWarps + warp) * GPW : 0);
+                const uint32_t mk = sm.mask[slot] >> (CLS == 0 ? (half * kBlendWarps + warp) * GPW : half * GPW);
 #pragma unroll
                 for (int g = 0; g < GPW; ++g) {
                     const bool hit = (mk >> g) & 1u;
                     const uint32_t b = __ballot_sync(0xffffffffu, hit);
                     const uint32_t at = n[g] + __popc(b & lanemask_lt);
                     if (hit) {
-                        sm.list[GPW * warp + g][at] = static_cast<uint16_t>(slot * 16u);
+                        sm.list[4 * warp + g][at] = static_cast<uint16_t>(slot * 16u);
                         if constexpr (log_mode)  // each step's Gaussian colour and opacity
                             reinterpret_cast<float4*>(sw.scratch + 256u * split_log_pos_unit())
                                 [static_cast<uint32_t>(GPW * warp + g) * sw.recs + n_logged[g] + at] = sm.rgba[slot];
@@ -2159,38 +2173,55 @@ __device__ __forceinline__ void blend_tile(const FrameParams& fp, const FrameBuf
                 n_logged[g] += n[g];
             }
         } else {
-            const uint32_t b0 = (__ballot_sync(0xffffffffu, mask[0] != 0u) >> (8 * grp)) & 0xffu;
-            const uint32_t b1 = (__ballot_sync(0xffffffffu, mask[1] != 0u) >> (8 * grp)) & 0xffu;
             const uint32_t lt8 = (1u << (lane & 7)) - 1u;
-            uint16_t* list = sm.list[GPW * warp + grp];
-            if (mask[0]) list[__popc(b0 & lt8)] = static_cast<uint16_t>((team_base + team_tid) * 16u);
-            if (mask[1]) list[__popc(b0) + __popc(b1 & lt8)] = static_cast<uint16_t>((team_base + TEAM + team_tid) * 16u);
-            n_mine = __popc(b0) + __popc(b1);
+            uint16_t* list = sm.list[4 * warp + grp];
+            n_mine = 0u;
+#pragma unroll
+            for (int h = 0; h < kBlendPerThread; ++h) {
+                const uint32_t b = (__ballot_sync(0xffffffffu, mask[h] != 0u) >> (8 * grp)) & 0xffu;
+                if (mask[h]) list[n_mine + __popc(b & lt8)] = static_cast<uint16_t>((team_base + h * TEAM + team_tid) * 16u);
+                n_mine += __popc(b);
+            }
             n_max = __reduce_max_sync(0xffffffffu, n_mine);
         }
-        uint16_t* list = sm.list[GPW * warp + grp];
+        uint16_t* list = sm.list[4 * warp + grp];
+        n_max = (n_max + EPS - 1u) & ~(EPS - 1u);
         for (uint32_t t = n_mine + lane % LPG; t < n_max; t += LPG) list[t] = kBlendDummy * 16;
         __syncwarp();
-        for (uint32_t t = 0; t < n_max; ++t) {
-            const uint32_t off = list[t];
-            auto lds = [&](const float4* a) { return *reinterpret_cast<const float4*>(reinterpret_cast<const char*>(a) + off); };
-            const float4 A = lds(sm.p1), B = lds(sm.p2), C = lds(sm.p4), c = lds(sm.rgba);
-            const float zmin = *reinterpret_cast<const float*>(reinterpret_cast<const char*>(sm.zmin) + (off >> 2));
-            float3 m[PX], d[PX];
-            float rcp[PX], alpha[PX];
-            float4 pm[PX];
-            bool frag[PX], cand = false;
+        // A step evaluates two pairs: one list entry for both pixels (PX 2), or two entries for one
+        // pixel, whose effects then follow in list order (PX 1: the second evaluation fills the
+        // latencies of the first; half items run where few warps are resident).
+        for (uint32_t t = 0; t < n_max; t += EPS) {
+            uint32_t off[EPS];
+            off[0] = list[t];
+            if constexpr (EPS == 2) off[1] = list[t + 1];
+            auto lds = [&](const float4* a, int e) {
+                return *reinterpret_cast<const float4*>(reinterpret_cast<const char*>(a) + off[e]);
+            };
+            float4 C[EPS], c[EPS];
+            float zmin[EPS];
+            float3 m[2], d[2];
+            float rcp[2], alpha[2];
+            float4 pm[2];
+            bool frag[2], cand = false;
+#pragma unroll
+            for (uint32_t e = 0; e < EPS; ++e) {
+                C[e] = lds(sm.p4, e);
+                c[e] = lds(sm.rgba, e);
+                zmin[e] = *reinterpret_cast<const float*>(reinterpret_cast<const char*>(sm.zmin) + (off[e] >> 2));
+            }
             // the fragment is evaluated for every lane and the tests only gate its effects (no
             // divergent exits; a lane that failed cannot contribute, whatever rcp / exp return)
             if constexpr (PX == 2) {
+                const float4 A = lds(sm.p1, 0), B = lds(sm.p2, 0);
                 // both pixels in packed arithmetic: m and d are the negatives of the scalar form's,
                 // (-a) b + (c d) for a b - (c d), which leaves num, den and cross(d, m) the same
-                const f32x2 X = both(__fmaf_rn(-C.x, pixel_x, A.x)), Y = both(__fmaf_rn(-C.y, pixel_x, A.y)),
-                            Z = both(__fmaf_rn(-C.z, pixel_x, A.z)), nX = both(__fmaf_rn(C.x, pixel_x, -A.x)),
-                            nY = both(__fmaf_rn(C.y, pixel_x, -A.y)), nZ = both(__fmaf_rn(C.z, pixel_x, -A.z)),
-                            nW = both(__fmaf_rn(C.w, pixel_x, -A.w));
-                const f32x2 yx = fma2(both(C.x), npixel_y, both(B.x)), yy = fma2(both(C.y), npixel_y, both(B.y)),
-                            yz = fma2(both(C.z), npixel_y, both(B.z)), yw = fma2(both(C.w), npixel_y, both(B.w));
+                const f32x2 X = both(__fmaf_rn(-C[0].x, pixel_x, A.x)), Y = both(__fmaf_rn(-C[0].y, pixel_x, A.y)),
+                            Z = both(__fmaf_rn(-C[0].z, pixel_x, A.z)), nX = both(__fmaf_rn(C[0].x, pixel_x, -A.x)),
+                            nY = both(__fmaf_rn(C[0].y, pixel_x, -A.y)), nZ = both(__fmaf_rn(C[0].z, pixel_x, -A.z)),
+                            nW = both(__fmaf_rn(C[0].w, pixel_x, -A.w));
+                const f32x2 yx = fma2(both(C[0].x), npixel_y, both(B.x)), yy = fma2(both(C[0].y), npixel_y, both(B.y)),
+                            yz = fma2(both(C[0].z), npixel_y, both(B.z)), yw = fma2(both(C[0].w), npixel_y, both(B.w));
                 const f32x2 mx = fma2(nW, yx, mul2(X, yw)), my = fma2(nW, yy, mul2(Y, yw)), mz = fma2(nW, yz, mul2(Z, yw));
                 const f32x2 dx = fma2(nY, yz, mul2(Z, yy)), dy = fma2(nZ, yx, mul2(X, yz)), dz = fma2(nX, yy, mul2(Y, yx));
                 const f32x2 num2 = fma2(mz, mz, fma2(mx, mx, mul2(my, my))), den2 = fma2(dz, dz, fma2(dx, dx, mul2(dy, dy)));
@@ -2201,13 +2232,13 @@ __device__ __forceinline__ void blend_tile(const FrameParams& fp, const FrameBuf
                 rcp[0] = 1.0f / den[0];
                 rcp[1] = 1.0f / den[1];
                 unpair(mul2(mul2(both(-0.5f), num2), pair(rcp[0], rcp[1])), e[0], e[1]);
-                unpair(mul2(both(c.w), pair(expf(e[0]), expf(e[1]))), alpha[0], alpha[1]);
+                unpair(mul2(both(c[0].w), pair(expf(e[0]), expf(e[1]))), alpha[0], alpha[1]);
                 alpha[0] = fminf(alpha[0], kMaxFragmentAlpha);
                 alpha[1] = fminf(alpha[1], kMaxFragmentAlpha);
                 const f32x2 al = pair(alpha[0], alpha[1]);
-                unpair(mul2(both(c.x), al), pm[0].x, pm[1].x);
-                unpair(mul2(both(c.y), al), pm[0].y, pm[1].y);
-                unpair(mul2(both(c.z), al), pm[0].z, pm[1].z);
+                unpair(mul2(both(c[0].x), al), pm[0].x, pm[1].x);
+                unpair(mul2(both(c[0].y), al), pm[0].y, pm[1].y);
+                unpair(mul2(both(c[0].z), al), pm[0].z, pm[1].z);
                 unpair(mx, m[0].x, m[1].x);
                 unpair(my, m[0].y, m[1].y);
                 unpair(mz, m[0].z, m[1].z);
@@ -2218,49 +2249,63 @@ __device__ __forceinline__ void blend_tile(const FrameParams& fp, const FrameBuf
                 for (int i = 0; i < 2; ++i) {
                     pm[i].w = alpha[i];
                     frag[i] = !(num[i] > lim[i]) && !(alpha[i] < kMinAlpha);
-                    cand = cand || (frag[i] && (log_mode || zmin < core[i][K - 1].depth));
+                    cand = cand || (frag[i] && (log_mode || zmin[0] < core[i][K - 1].depth));
                 }
             } else {
-                const float3 nx = make_float3(__fmaf_rn(-C.x, pixel_x, A.x), __fmaf_rn(-C.y, pixel_x, A.y), __fmaf_rn(-C.z, pixel_x, A.z));
-                const float wx = __fmaf_rn(-C.w, pixel_x, A.w);
-                const float3 ny = make_float3(__fmaf_rn(-C.x, pixel_y[0], B.x), __fmaf_rn(-C.y, pixel_y[0], B.y),
-                                              __fmaf_rn(-C.z, pixel_y[0], B.z));
-                const float wy = __fmaf_rn(-C.w, pixel_y[0], B.w);
-                m[0] = make_float3(mulsub(wx, ny.x, nx.x, wy), mulsub(wx, ny.y, nx.y, wy), mulsub(wx, ny.z, nx.z, wy));
-                d[0] = cross_fma(nx, ny);
-                const float num = dot_xyz(m[0], m[0]), den = dot_xyz(d[0], d[0]);
-                const bool in = !(num > kMaxCutoffSq * den);
-                rcp[0] = 1.0f / den;
-                alpha[0] = fminf(c.w * expf(-0.5f * num * rcp[0]), kMaxFragmentAlpha);
-                frag[0] = in && !(alpha[0] < kMinAlpha);
-                cand = frag[0] && zmin < core[0][K - 1].depth;
-                pm[0] = make_float4(c.x * alpha[0], c.y * alpha[0], c.z * alpha[0], alpha[0]);
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const float4 A = lds(sm.p1, e), B = lds(sm.p2, e);
+                    const float4 Ce = C[e % EPS], ce = c[e % EPS];
+                    const float3 nx = make_float3(__fmaf_rn(-Ce.x, pixel_x, A.x), __fmaf_rn(-Ce.y, pixel_x, A.y), __fmaf_rn(-Ce.z, pixel_x, A.z));
+                    const float wx = __fmaf_rn(-Ce.w, pixel_x, A.w);
+                    const float3 ny = make_float3(__fmaf_rn(-Ce.x, pixel_y[0], B.x), __fmaf_rn(-Ce.y, pixel_y[0], B.y),
+                                                  __fmaf_rn(-Ce.z, pixel_y[0], B.z));
+                    const float wy = __fmaf_rn(-Ce.w, pixel_y[0], B.w);
+                    m[e] = make_float3(mulsub(wx, ny.x, nx.x, wy), mulsub(wx, ny.y, nx.y, wy), mulsub(wx, ny.z, nx.z, wy));
+                    d[e] = cross_fma(nx, ny);
+                    const float num = dot_xyz(m[e], m[e]), den = dot_xyz(d[e], d[e]);
+                    const bool in = !(num > kMaxCutoffSq * den);
+                    rcp[e] = 1.0f / den;
+                    alpha[e] = fminf(ce.w * expf(-0.5f * num * rcp[e]), kMaxFragmentAlpha);
+                    frag[e] = in && !(alpha[e] < kMinAlpha);
+                    cand = cand || (frag[e] && zmin[e % EPS] < core[0][K - 1].depth);
+                    pm[e] = make_float4(ce.x * alpha[e], ce.y * alpha[e], ce.z * alpha[e], alpha[e]);
+                }
             }
             // The depth matters only to a fragment that may enter the core: alpha >= 1/20 and a
             // depth below the core's last.  `zmin` bounds it from below, so that once the near
             // Gaussians are in, almost no step evaluates it (a warp-uniform branch).
-            float logged_depth[PX] = {};
+            float logged_depth[2] = {};
+            auto accumulate = [&](int i) {
+                if (frag[i]) {
+                    const int px = PX == 2 ? i : 0;
+                    const float pt = 1.0f - pm[i].w;
+                    tail[px] += pm[i];
+                    tail_T[px] *= pt;
+                }
+            };
             if (__any_sync(0xffffffffu, cand)) {
 #pragma unroll
-                for (int i = 0; i < PX; ++i) {
+                for (int i = 0; i < 2; ++i) {
+                    const int px = PX == 2 ? i : 0;
                     const float3 e = cross_fma(d[i], m[i]);
                     const float3 ep = make_float3(__fmul_rn(e.x, rcp[i]), __fmul_rn(e.y, rcp[i]), __fmul_rn(e.z, rcp[i]));
-                    const float depth = __fadd_rn(dot_xyz(xyz(C), ep), C.w);
+                    const float depth = __fadd_rn(dot_xyz(xyz(C[i % EPS]), ep), C[i % EPS].w);
                     if constexpr (log_mode) logged_depth[i] = depth;
                     if constexpr (!log_mode) {
-                        const bool ins = frag[i] && alpha[i] >= kMinAlphaCore && depth < core[i][K - 1].depth;
+                        const bool ins = frag[i] && alpha[i] >= kMinAlphaCore && depth < core[px][K - 1].depth;
                         if (__any_sync(0xffffffffu, ins)) {  // lanes without an insertion: FLT_MAX changes nothing
                             if constexpr (SEG == 1) {
                                 if (ins && sw.mode == 2) {  // recorded; the merge decides what it does
-                                    if (n_rec[i] < static_cast<uint32_t>(sw.recs)) {
-                                        const uint32_t at = n_rec[i] * NT + tid + i * kBlendThreads;
+                                    if (n_rec[px] < static_cast<uint32_t>(sw.recs)) {
+                                        const uint32_t at = n_rec[px] * NT + tid + i * kBlendThreads;
                                         reinterpret_cast<float*>(sw.scratch + 6 * 4 * NT)[at] = depth;
                                         reinterpret_cast<float4*>(sw.scratch + (6 + sw.recs) * 4 * NT)[at] = pm[i];
                                     }
-                                    ++n_rec[i];
+                                    ++n_rec[px];
                                 }
                             }
-                            float4 ev = unpack_rgba(core_insert<K>(core[i], ins ? depth : 3.402823466e+38f, pm[i]));
+                            float4 ev = unpack_rgba(core_insert<K>(core[px], ins ? depth : 3.402823466e+38f, pm[i]));
                             if constexpr (SEG == 1) {
                                 if (sw.mode == 2) ev = make_float4(0.0f, 0.0f, 0.0f, 0.0f);  // adds nothing below
                             }
@@ -2278,14 +2323,8 @@ __device__ __forceinline__ void blend_tile(const FrameParams& fp, const FrameBuf
                     for (int i = 0; i < PX; ++i) fr[8 * i] = make_float2(frag[i] ? alpha[i] : -1.0f, logged_depth[i]);
                 }
             } else {
-#pragma unroll
-                for (int i = 0; i < PX; ++i) {
-                    if (frag[i]) {
-                        const float pt = 1.0f - pm[i].w;
-                        tail[i] += pm[i];
-                        tail_T[i] *= pt;
-                    }
-                }
+                accumulate(0);
+                accumulate(1);
             }
         }
     }
@@ -2532,7 +2571,11 @@ __global__ void __launch_bounds__(kBlendThreads, blend_blocks(K)) blend_kernel(F
             blend_tile<K, RW, 0, 1>(fp, fb, item, static_cast<int>(kind - kItemHalf), true, sm);
         } else if (kind == kItemLow) {
             const uint32_t i = (item & kItemNumberMask) * kLowTiles + warp;
-            if (i < n_low) blend_tile<K, RW, 1, 2>(fp, fb, runs[i], 0, true, sm);
+            if (i < n_low) {
+                const uint32_t tile = runs[i], part = tile >> kItemKindShift;
+                if (part == kItemFull) blend_tile<K, RW, 1, 2>(fp, fb, tile, 0, true, sm);
+                else blend_tile<K, RW, 1, 1>(fp, fb, tile, static_cast<int>(part - kItemHalf), true, sm);
+            }
         } else {
             const uint32_t i0 = (item & kItemNumberMask) * kQuarterTiles + 4 * warp, i = i0 + (lane >> 3);
             if (i0 < n_quarter)

@@ -152,7 +152,7 @@ struct FrameBuffers {
     uint32_t* work_masked;    // [V][max_large] masked large tiles
     uint32_t* counters;       // [kCounterWords]: work counters, then the work-order buckets
     uint32_t* work_order[2];  // [0]: [2*V*max_large] the blend's block items, longest first;
-                              // [1]: [V*max_large] the tiles of its periphery and quarter items
+                              // [1]: [2*V*max_large] the tiles of its periphery and quarter items
     // Onesweep sort state (null: the three-kernel sort, which needs sort_hist/sort_digit_tot):
     uint32_t* sort_ghist;     // [V][kSortMaxPasses][256] digit counts of every pass (create fills)
     uint32_t* sort_look;      // [V][kSortMaxPasses][sort_tiles][256] look-back words
