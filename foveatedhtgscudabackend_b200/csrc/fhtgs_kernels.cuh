@@ -775,6 +775,12 @@ __device__ __forceinline__ void count_key(uint32_t* s_hist, int passes, uint32_t
     for (int p = 0; p < passes; ++p) atomicAdd(&s_hist[p * kSortBins + ((key >> (p * kSortRadixBits)) & (kSortBins - 1))], 1u);
 }
 
+// Blocks of the creation over all views; each loops over chunks of 256 Gaussians, so that the
+// digit counts of a frame of many views reach the few global counters once per block instead of
+// once per chunk (12 views of 1M: scan + create 0.483 -> 0.295 ms; stereo 1M 0.129 -> 0.125 ms;
+// a quarter as many blocks leave the uneven chunks unbalanced: 0.157 ms stereo).
+constexpr int kCreateBlocks = 32 * 148;
+
 template <typename KeyT>
 __global__ void __launch_bounds__(kPrimBlock) create_instances_kernel(FrameParams fp, FrameBuffers fb) {
     __shared__ uint32_t s_warp[33];
@@ -785,20 +791,13 @@ __global__ void __launch_bounds__(kPrimBlock) create_instances_kernel(FrameParam
     __shared__ ushort4 s_big_b[kBigList];
     const int v = blockIdx.y;
     const ViewParams& vp = fb.views[v];
-    const int i = blockIdx.x * kPrimBlock + threadIdx.x;
     const size_t N = static_cast<size_t>(fp.n_prims);
-    const size_t o = static_cast<size_t>(v) * N + i;
-    const uint32_t nv = i < fp.n_prims ? fb.n_vis[o] : 0u;
-    uint32_t tot;
-    const uint32_t local = block_excl_scan<uint32_t>(nv, tot, s_warp);
-    const uint32_t off = fb.block_sums[static_cast<size_t>(v) * fp.n_blocks_prim + blockIdx.x] + local;
     const uint64_t lim = static_cast<uint64_t>(fp.cap);
     KeyT* keys = reinterpret_cast<KeyT*>(fb.keys[0]) + static_cast<size_t>(v) * fp.cap;
     uint32_t* vals = fb.vals[0] + static_cast<size_t>(v) * fp.cap;
     const uint32_t glw = static_cast<uint32_t>(vp.glw);
     const bool onesweep = fb.sort_ghist != nullptr;
     const int passes = sort_passes(fp);
-    if (threadIdx.x == 0) s_big_n = 0;
     if (onesweep) {
         for (int k = threadIdx.x; k < kSortMaxPasses * kSortBins; k += kPrimBlock) s_dhist[k] = 0u;
         // look-back words of this view's tiles: [pass][tile][digit], tiles of the stored count
@@ -812,77 +811,86 @@ __global__ void __launch_bounds__(kPrimBlock) create_instances_kernel(FrameParam
                  k += static_cast<uint64_t>(gridDim.x) * kPrimBlock)
                 look[p * pass_stride + k] = 0u;
     }
-    __syncthreads();
-    if (nv > 0) {
-        const ushort4 b = fb.bounds[o];
-        const uint32_t bw = static_cast<uint32_t>(b.y - b.x);
-        const uint32_t cnt = static_cast<uint32_t>(b.w - b.z) * bw;
-        if (cnt <= kSeqTiles) {
-            uint64_t w = off;
-            const uint64_t end = static_cast<uint64_t>(off) + nv;
-            for (uint32_t ty = b.z; ty < b.w && w < end; ++ty) {  // row-major over the bounds
-                const uint32_t row = ty * glw;
-                for (uint32_t tx = b.x; tx < b.y && w < end; ++tx) {
-                    const uint32_t tile = row + tx;
-                    if (!tile_visible(vp.vis_mask, tile)) continue;
-                    if (w < lim) {
-                        keys[w] = static_cast<KeyT>(tile);
-                        vals[w] = static_cast<uint32_t>(i);
-                        if (onesweep) count_key(s_dhist, passes, tile);
+    for (int chunk = blockIdx.x; chunk < fp.n_blocks_prim; chunk += gridDim.x) {
+        const int i = chunk * kPrimBlock + threadIdx.x;
+        const size_t o = static_cast<size_t>(v) * N + i;
+        const uint32_t nv = i < fp.n_prims ? fb.n_vis[o] : 0u;
+        if (threadIdx.x == 0) s_big_n = 0;
+        uint32_t tot;
+        const uint32_t local = block_excl_scan<uint32_t>(nv, tot, s_warp);  // (its barriers publish s_big_n and s_dhist)
+        const uint32_t off = fb.block_sums[static_cast<size_t>(v) * fp.n_blocks_prim + chunk] + local;
+        if (nv > 0) {
+            const ushort4 b = fb.bounds[o];
+            const uint32_t bw = static_cast<uint32_t>(b.y - b.x);
+            const uint32_t cnt = static_cast<uint32_t>(b.w - b.z) * bw;
+            if (cnt <= kSeqTiles) {
+                uint64_t w = off;
+                const uint64_t end = static_cast<uint64_t>(off) + nv;
+                for (uint32_t ty = b.z; ty < b.w && w < end; ++ty) {  // row-major over the bounds
+                    const uint32_t row = ty * glw;
+                    for (uint32_t tx = b.x; tx < b.y && w < end; ++tx) {
+                        const uint32_t tile = row + tx;
+                        if (!tile_visible(vp.vis_mask, tile)) continue;
+                        if (w < lim) {
+                            keys[w] = static_cast<KeyT>(tile);
+                            vals[w] = static_cast<uint32_t>(i);
+                            if (onesweep) count_key(s_dhist, passes, tile);
+                        }
+                        ++w;
                     }
-                    ++w;
                 }
+                // a visibility area table that counts more tiles than the mask holds leaves slots
+                // over: they get sentinels that the range and blend stages skip
+                for (; w < end && w < lim; ++w) {
+                    keys[w] = static_cast<KeyT>(~KeyT(0));
+                    vals[w] = kNoPrimitive;
+                    if (onesweep) count_key(s_dhist, passes, static_cast<KeyT>(~KeyT(0)));
+                }
+            } else {
+                const uint32_t slot = atomicAdd(&s_big_n, 1u);
+                s_big_prim[slot] = static_cast<uint32_t>(i);
+                s_big_off[slot] = off;
+                s_big_b[slot] = b;
             }
-            // a visibility area table that counts more tiles than the mask holds leaves slots
-            // over: they get sentinels that the range and blend stages skip
-            for (; w < end && w < lim; ++w) {
+        }
+        __syncthreads();
+        // Large bounds: one warp per Gaussian (eight at a time), 32 tiles per step in row-major
+        // bounds order, a ballot of the per-tile visibility giving each visible tile its slot; no
+        // block barrier, so the warps do not wait for one another's Gaussians.
+        const uint32_t n_big = s_big_n;
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        const uint32_t lanemask_lt = (1u << lane) - 1u;
+        for (uint32_t q = warp; q < n_big; q += kPrimBlock / 32) {
+            const uint32_t prim = s_big_prim[q];
+            const ushort4 bb = s_big_b[q];
+            const uint32_t bw = static_cast<uint32_t>(bb.y - bb.x);
+            const uint32_t cnt = static_cast<uint32_t>(bb.w - bb.z) * bw;
+            uint64_t w0 = s_big_off[q];
+            const uint64_t end = w0 + fb.n_vis[static_cast<size_t>(v) * N + prim];
+            for (uint32_t base = 0; base < cnt; base += 32) {
+                const uint32_t k = base + lane;
+                uint32_t tile = 0;
+                bool c = false;
+                if (k < cnt) {
+                    tile = (bb.z + k / bw) * glw + bb.x + k % bw;
+                    c = tile_visible(vp.vis_mask, tile);
+                }
+                const uint32_t vote = __ballot_sync(0xffffffffu, c);
+                const uint64_t w = w0 + __popc(vote & lanemask_lt);
+                if (c && w < lim && w < end) {
+                    keys[w] = static_cast<KeyT>(tile);
+                    vals[w] = prim;
+                    if (onesweep) count_key(s_dhist, passes, tile);
+                }
+                w0 += __popc(vote);
+            }
+            for (uint64_t w = w0 + lane; w < end && w < lim; w += 32) {  // see above
                 keys[w] = static_cast<KeyT>(~KeyT(0));
                 vals[w] = kNoPrimitive;
                 if (onesweep) count_key(s_dhist, passes, static_cast<KeyT>(~KeyT(0)));
             }
-        } else {
-            const uint32_t slot = atomicAdd(&s_big_n, 1u);
-            s_big_prim[slot] = static_cast<uint32_t>(i);
-            s_big_off[slot] = off;
-            s_big_b[slot] = b;
         }
-    }
-    __syncthreads();
-    // Large bounds: one warp per Gaussian (eight at a time), 32 tiles per step in row-major
-    // bounds order, a ballot of the per-tile visibility giving each visible tile its slot; no
-    // block barrier, so the warps do not wait for one another's Gaussians.
-    const uint32_t n_big = s_big_n;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t lanemask_lt = (1u << lane) - 1u;
-    for (uint32_t q = warp; q < n_big; q += kPrimBlock / 32) {
-        const uint32_t prim = s_big_prim[q];
-        const ushort4 bb = s_big_b[q];
-        const uint32_t bw = static_cast<uint32_t>(bb.y - bb.x);
-        const uint32_t cnt = static_cast<uint32_t>(bb.w - bb.z) * bw;
-        uint64_t w0 = s_big_off[q];
-        const uint64_t end = w0 + fb.n_vis[static_cast<size_t>(v) * N + prim];
-        for (uint32_t base = 0; base < cnt; base += 32) {
-            const uint32_t k = base + lane;
-            uint32_t tile = 0;
-            bool c = false;
-            if (k < cnt) {
-                tile = (bb.z + k / bw) * glw + bb.x + k % bw;
-                c = tile_visible(vp.vis_mask, tile);
-            }
-            const uint32_t vote = __ballot_sync(0xffffffffu, c);
-            const uint64_t w = w0 + __popc(vote & lanemask_lt);
-            if (c && w < lim && w < end) {
-                keys[w] = static_cast<KeyT>(tile);
-                vals[w] = prim;
-                if (onesweep) count_key(s_dhist, passes, tile);
-            }
-            w0 += __popc(vote);
-        }
-        for (uint64_t w = w0 + lane; w < end && w < lim; w += 32) {  // see above
-            keys[w] = static_cast<KeyT>(~KeyT(0));
-            vals[w] = kNoPrimitive;
-            if (onesweep) count_key(s_dhist, passes, static_cast<KeyT>(~KeyT(0)));
-        }
+        __syncthreads();  // the big list is reused
     }
     if (onesweep) {
         __syncthreads();
@@ -894,7 +902,8 @@ __global__ void __launch_bounds__(kPrimBlock) create_instances_kernel(FrameParam
 
 int launch_create(const FrameParams& fp, const FrameBuffers& fb, cudaStream_t s) {
     if (fp.n_blocks_prim == 0) return 0;
-    dim3 grid(fp.n_blocks_prim, fp.n_views);
+    const int per_view = (kCreateBlocks + fp.n_views - 1) / fp.n_views;
+    dim3 grid(fp.n_blocks_prim < per_view ? fp.n_blocks_prim : per_view, fp.n_views);
     if (fp.key_u32) create_instances_kernel<uint32_t><<<grid, kPrimBlock, 0, s>>>(fp, fb);
     else create_instances_kernel<uint16_t><<<grid, kPrimBlock, 0, s>>>(fp, fb);
     return 1;
