@@ -971,7 +971,7 @@ fhtgs_status fhtgs_autotune(fhtgs_context ctx, const fhtgs_primitives* prims, co
     constexpr int kStageSort = 3, kStageBlend = 5;
     fhtgs_tuning cur = start;
     float best_stage = 3.4e38f, frame = 0.0f, stage = 0.0f;
-    // blend: warp rectangle x persistent blocks per SM
+    // blend: group rectangle x most persistent blocks per SM
     fhtgs_tuning win = cur;
     for (int w : kBlendRowChoices) {
         for (int b : {0, 3, 2}) {
