@@ -334,7 +334,7 @@ fhtgs_status fhtgs_context_set_blend_split(fhtgs_context ctx, float segment_shar
  * and each step's Gaussian colour), and the last segment of a tile replays the log with the
  * walk's own K-buffer and tail steps, so the operations and their order are those of the serial
  * walk: images bit-identical to the default path.  The logs share one pool of `log_bytes`
- * (0 = 8 GiB; about 2.2 KB per list entry of a split tile); a tile whose segments do
+ * (0 = 8 GiB; about 2.3 KB per list entry of a split tile); a tile whose segments do
  * not fit it is blended whole.  The share set by fhtgs_context_set_blend_split applies. */
 fhtgs_status fhtgs_context_set_blend_split_exact(fhtgs_context ctx, int32_t exact, int64_t log_bytes);
 /* The last frame's split blend: tiles split, segments blended, tiles blended whole after a record
