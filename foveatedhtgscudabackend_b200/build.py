@@ -40,7 +40,8 @@ UNITS = [
     ("fhtgs_server.cu", []),
     ("fhtgs_group.cu", []),
 ]
-HEADERS = ["fhtgs_types.cuh", "fhtgs_math.cuh", "fhtgs_kernels.cuh", "fhtgs_internal.h", "fhtgs_route.h"]
+HEADERS = ["fhtgs_types.cuh", "fhtgs_math.cuh", "fhtgs_kernels.cuh", "fhtgs_internal.h", "fhtgs_route.h",
+           "fhtgs_order.h"]
 
 
 def nvcc() -> str:

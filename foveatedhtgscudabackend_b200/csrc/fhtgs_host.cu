@@ -206,7 +206,7 @@ Layout plan(int V, int64_t N, int nbp, int64_t cap, int key_bytes, int sort_tile
     L.off_wm = take(4ull * V * max_large);
     L.off_ctr = take(4ull * kCounterWords);
     L.off_order0 = take(8ull * V * max_large);
-    L.off_order1 = take(8ull * V * max_large);
+    L.off_order1 = take(10ull * V * max_large);
     L.off_ghist = take(4ull * V * kSortMaxPasses * kSortBins);
     L.off_look = take(4ull * V * kSortMaxPasses * sort_tiles * kSortBins);
     L.off_ticket = take(4ull * V * kSortMaxPasses);

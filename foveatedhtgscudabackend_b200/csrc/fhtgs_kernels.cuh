@@ -1324,27 +1324,9 @@ int launch_ranges(const FrameParams& fp, const FrameBuffers& fb, int n_sms, cuda
 }
 
 // ------------------------------------------------------------------------------------------
-// work ordering for the persistent blend (bucketed longest-processing-time first)
-// One list of block items, longest estimated duration first, so that the serial walks of the
-// long lists start early and the short ones fill the end:
-//   full    a full-resolution tile, two pixels a thread
-//   half    the upper or lower half of a full-resolution tile, one pixel a thread: the tiles
-//           whose walk alone would outlast the frame's mean work per block
-//   low     four periphery tiles, or halves of them, one per warp
-//   quarter sixteen ring-mode quarter tiles, four per warp
-// An item word is kind << 29 | view << 21 | index into the view's work_full list, or kind << 29 |
-// item number for the last two, whose tiles lie in work_order[1] (the same word, with the index
-// into work_low), longest first: the periphery tiles of all views, then the quarter tiles.
+// work ordering for the persistent blend (bucketed longest-processing-time first).
+// The items, their words and their places: fhtgs_order.h.
 // ------------------------------------------------------------------------------------------
-constexpr uint32_t kItemFull = 0u, kItemHalf = 1u /* and 2 */, kItemLow = 3u, kItemQuarter = 4u;
-constexpr int kItemKindShift = 29, kItemViewShift = 21;
-constexpr uint32_t kItemIndexMask = (1u << kItemViewShift) - 1u;
-constexpr uint32_t kItemNumberMask = (1u << kItemKindShift) - 1u;
-__device__ __forceinline__ int item_view(uint32_t packed) { return static_cast<int>((packed >> kItemViewShift) & 255u); }
-__device__ __forceinline__ uint32_t item_index(uint32_t packed) { return packed & kItemIndexMask; }
-// Tiles (or halves) of a low / quarter item.
-constexpr uint32_t kLowTiles = 4, kQuarterTiles = 16;
-
 // Estimated duration of an item in list entries of a full item: per entry of its (longest) list,
 // plus the item's fixed cost.  Measured at five blocks per SM: 168 ns per entry of a full item and
 // 90 of a half item (stereo frame), 144 and 208 of a full and a periphery item (6M Gaussians,
@@ -1401,6 +1383,13 @@ __device__ __forceinline__ int item_tile(const FrameParams& fp, const FrameBuffe
     return !low ? 2 : static_cast<uint32_t>(idx) < st.n_periphery_large ? 1 : 0;
 }
 
+// [V][max_large] order_word of each tile (full-resolution, periphery, quarter), behind the runs (no
+// field of its own: the preprocess takes FrameBuffers too, and its arithmetic depends on the
+// layout of its parameters).
+__device__ __forceinline__ uint16_t* order_decisions(const FrameParams& fp, const FrameBuffers& fb) {
+    return reinterpret_cast<uint16_t*>(fb.work_order[1] + 2 * static_cast<size_t>(fp.n_views) * fp.max_large);
+}
+
 // Estimated duration of a tile's item (class 2: full or half), see kCostHalf.
 __device__ __forceinline__ float item_cost(int cls, uint32_t len, bool halves) {
     const float c = cls == 2 ? 1.0f : cls == 1 ? kCostLow : kCostQuarter;
@@ -1410,8 +1399,6 @@ __device__ __forceinline__ float item_cost(int cls, uint32_t len, bool halves) {
 __device__ __forceinline__ bool blend_halves(int cls, uint32_t len, uint32_t half_len) {
     return cls == 2 ? len > half_len : cls == 1 && kCostLow * static_cast<float>(len) > static_cast<float>(half_len);
 }
-// Its bucket: class above duration bucket.
-__device__ __forceinline__ int item_bucket(int cls, float cost) { return cls * kCostBuckets + cost_bucket(cost); }
 
 // List length above which a full-resolution tile is blended as two half items.
 __device__ __forceinline__ uint32_t half_threshold(const FrameParams& fp, const FrameBuffers& fb, int n_sms) {
@@ -1502,13 +1489,18 @@ __global__ void __launch_bounds__(256) order_hist_kernel(FrameParams fp, FrameBu
                 }
             }
             sp.of[static_cast<size_t>(v) * fp.max_large + j] = tag;
-            if (tag != ~0u) continue;
+            if (tag != ~0u) {
+                order_decisions(fp, fb)[static_cast<size_t>(v) * fp.max_large + j] = kOrderSplit;
+                continue;
+            }
         }
         const bool halves = blend_halves(cls, len, half_len);
         const float cost = item_cost(cls, len, halves);
         longest = fmaxf(longest, cost);
         cost_sum += cost * (halves ? 2.0f : 1.0f) / static_cast<float>(cls == 2 ? 1u : cls == 1 ? kLowTiles : kQuarterTiles);
-        atomicAdd(&hist[item_bucket(cls, cost)], halves ? 2u : 1u);
+        const uint16_t word = order_word(cls * kCostBuckets + cost_bucket(cost), halves);
+        order_decisions(fp, fb)[static_cast<size_t>(v) * fp.max_large + j] = word;
+        atomicAdd(&hist[order_bucket(word)], order_entries(word));
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -1536,21 +1528,20 @@ __global__ void __launch_bounds__(256) order_hist_kernel(FrameParams fp, FrameBu
 // Tiles go to their bucket's run in rounds of blockDim.x: a block counts its round's entries per
 // bucket in shared memory (each tile's rank among them), reserves one contiguous place per bucket
 // with a single global atomic, and writes them there.  (One global atomic per tile made the few
-// heavily used buckets' cursors a serial bottleneck.)  The place of a block item in the merged
-// list is its place in its own class plus the items of the other classes in longer buckets (equal
-// buckets: full, low, quarter).  The order inside a bucket follows the reservations; it changes
-// the schedule, never a pixel.
+// heavily used buckets' cursors a serial bottleneck.)  The buckets are those that order_hist_kernel
+// counted and stored: an estimate made again here could round differently (the compiler contracts
+// each kernel by itself), and a tile counted in one bucket and written in another overruns a run,
+// drops a tile and leaves an item word of an earlier frame.  The order inside a bucket follows the
+// reservations; it changes the schedule, never a pixel.
 __global__ void __launch_bounds__(256) order_scatter_kernel(FrameParams fp, FrameBuffers fb, SplitArgs sp, int n_sms,
                                                             int max_per_sm) {
     __shared__ int pre[kMaxOrderViews];
-    __shared__ uint32_t base[kOrderBuckets + 1];  // entries in higher buckets (of this and higher classes)
+    __shared__ uint32_t base[kOrderBuckets];  // entries in higher buckets (of this and higher classes)
     __shared__ uint32_t s_cnt[kOrderBuckets];
     __shared__ uint32_t s_warp[33];
-    __shared__ uint32_t s_half_len;
     const int total = items_prefix(fp, fb, pre);
     const uint32_t* gh = fb.counters + kCtrHist;
     uint32_t* cursor = fb.counters + kCtrHist + kOrderBuckets;
-    if (threadIdx.x == 0) s_half_len = half_threshold(fp, fb, n_sms);
     uint32_t all;
     {  // a block scan in descending bucket order, two buckets a thread
         static_assert(kOrderBuckets <= 2 * 256, "two buckets per thread of a 256-thread block");
@@ -1562,78 +1553,42 @@ __global__ void __launch_bounds__(256) order_scatter_kernel(FrameParams fp, Fram
         if (p1 < kOrderBuckets) base[kOrderBuckets - 1 - p1] = e + c0;
     }
     __syncthreads();
-    const uint32_t half_len = s_half_len;
-    const uint32_t n_full = base[2 * kCostBuckets - 1];  // entries above the periphery class
-    const uint32_t n_low = base[kCostBuckets - 1] - n_full, n_quarter = all - n_full - n_low;
+    const OrderTotals totals(base, all);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        fb.counters[kCtrItems] = n_full + (n_low + kLowTiles - 1) / kLowTiles + (n_quarter + kQuarterTiles - 1) / kQuarterTiles;
-        fb.counters[kCtrLow] = n_low;
-        fb.counters[kCtrQuarter] = n_quarter;
+        fb.counters[kCtrItems] = totals.items();
+        fb.counters[kCtrLow] = totals.low;
+        fb.counters[kCtrQuarter] = totals.quarter;
         const float u = __uint_as_float(fb.counters[kCtrLongest]) * static_cast<float>(n_sms) /
                         fmaxf(__uint_as_float(fb.counters[kCtrCost]), 1.0f);
         fb.counters[kCtrBlocks] = static_cast<uint32_t>(n_sms) * blocks_per_sm(u, static_cast<uint32_t>(max_per_sm));
     }
-    // entries of a class in duration buckets >= d (d = kCostBuckets: none)
-    auto at_least = [&](int cls, int d) {
-        const uint32_t start = cls == 2 ? 0u : cls == 1 ? n_full : n_full + n_low;
-        if (d >= kCostBuckets) return 0u;
-        const int k = cls * kCostBuckets + d;
-        return (k > 0 ? base[k - 1] : all) - start;
-    };
-    auto low_items = [&](int d) { return (at_least(1, d) + kLowTiles - 1) / kLowTiles; };
-    auto quarter_items = [&](int d) { return (at_least(0, d) + kQuarterTiles - 1) / kQuarterTiles; };
-    uint32_t* out = fb.work_order[0];
-    uint32_t* runs = fb.work_order[1];
     for (int g0 = blockIdx.x * blockDim.x; g0 < total; g0 += gridDim.x * blockDim.x) {
         for (int k = threadIdx.x; k < kOrderBuckets; k += blockDim.x) s_cnt[k] = 0;
         __syncthreads();
         const int g = g0 + static_cast<int>(threadIdx.x);
-        int b = -1, cls = 0;
-        bool halves = false;
+        uint16_t word = kOrderSplit;
         uint32_t packed = 0, local = 0;
         if (g < total) {
             int v, j;
             item_of(g, pre, fp.n_views, v, j);
-            uint32_t len;
-            cls = item_tile(fp, fb, v, j, len, packed);
-            halves = blend_halves(cls, len, half_len);
-            b = item_bucket(cls, item_cost(cls, len, halves));
-            if (sp.of != nullptr && sp.share > 0.0f && cls == 2) {
+            word = order_decisions(fp, fb)[static_cast<size_t>(v) * fp.max_large + j];
+            const FrameStatus& st = fb.status[v];
+            const uint32_t n_full = st.n_fovea_large + st.n_blended_large, idx = static_cast<uint32_t>(j);
+            packed = (static_cast<uint32_t>(v) << kItemViewShift) | (idx < n_full ? idx : idx - n_full);
+            if (word != kOrderSplit) {
+                local = atomicAdd(&s_cnt[order_bucket(word)], order_entries(word));
+            } else {  // a split tile: its segments go to the split list
                 const uint32_t tag = sp.of[static_cast<size_t>(v) * fp.max_large + j];
-                if (tag != ~0u) {  // a split tile: its segments go to the split list
-                    const uint32_t seg0 = tag & 0x0fffffffu, S = tag >> 28;
-                    for (uint32_t k = 0; k < S; ++k) sp.list[seg0 + k] = make_uint2(packed, tag);
-                    b = -1;
-                }
+                const uint32_t seg0 = tag & 0x0fffffffu, S = tag >> 28;
+                for (uint32_t k = 0; k < S; ++k) sp.list[seg0 + k] = make_uint2(packed, tag);
             }
-            if (b >= 0) local = atomicAdd(&s_cnt[b], halves ? 2u : 1u);
         }
         __syncthreads();
         for (int k = threadIdx.x; k < kOrderBuckets; k += blockDim.x)
             if (s_cnt[k]) s_cnt[k] = atomicAdd(&cursor[k], s_cnt[k]);
         __syncthreads();
-        if (b >= 0) {
-            const uint32_t at = base[b] + s_cnt[b] + local;  // place among all entries, classes one after the other
-            const int d = b - cls * kCostBuckets;
-            if (cls == 2) {
-                const uint32_t place = at + low_items(d + 1) + quarter_items(d + 1);
-                if (halves) {
-                    out[place] = (kItemHalf << kItemKindShift) | packed;
-                    out[place + 1] = ((kItemHalf + 1u) << kItemKindShift) | packed;
-                } else {
-                    out[place] = (kItemFull << kItemKindShift) | packed;
-                }
-            } else {
-                const uint32_t kind = halves ? kItemHalf : kItemFull;
-                runs[at - n_full] = (kind << kItemKindShift) | packed;
-                if (halves) runs[at - n_full + 1] = ((kind + 1u) << kItemKindShift) | packed;
-                const uint32_t per = cls == 1 ? kLowTiles : kQuarterTiles, k = at - n_full - (cls == 1 ? 0u : n_low);
-                const uint32_t first = (k + per - 1) / per * per;
-                if (first < k + (halves ? 2u : 1u))  // the first tile (or half) of an item
-                    out[first / per + at_least(2, d) + (cls == 1 ? quarter_items(d + 1) : low_items(d))] =
-                        ((cls == 1 ? kItemLow : kItemQuarter) << kItemKindShift) | (first / per);
-            }
-        }
+        if (word != kOrderSplit)
+            totals.put(word, base[order_bucket(word)] + s_cnt[order_bucket(word)] + local, packed, fb.work_order[0], fb.work_order[1]);
         __syncthreads();  // the counts are cleared for the next round
     }
 }

@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "fhtgs_order.h"
+
 namespace fhtgs {
 
 // Renderer constants; identical values to rasterization/include/config.h:13-45 of the
@@ -152,16 +154,14 @@ struct FrameBuffers {
     uint32_t* work_masked;    // [V][max_large] masked large tiles
     uint32_t* counters;       // [kCounterWords]: work counters, then the work-order buckets
     uint32_t* work_order[2];  // [0]: [2*V*max_large] the blend's block items, longest first;
-                              // [1]: [2*V*max_large] the tiles of its periphery and quarter items
+                              // [1]: [2*V*max_large] the tiles of its periphery and quarter items,
+                              // then the tiles' decisions (order_decisions)
     // Onesweep sort state (null: the three-kernel sort, which needs sort_hist/sort_digit_tot):
     uint32_t* sort_ghist;     // [V][kSortMaxPasses][256] digit counts of every pass (create fills)
     uint32_t* sort_look;      // [V][kSortMaxPasses][sort_tiles][256] look-back words
     uint32_t* sort_ticket;    // [V][kSortMaxPasses] tiles handed out so far
 };
 
-// Work ordering: tiles are bucketed by class and by estimated duration in quarter octaves.
-constexpr int kCostBuckets = 130;                     // per tile class
-constexpr int kOrderBuckets = 3 * kCostBuckets;       // quarter, periphery, full-resolution
 // counters: the blend's next block item; the split blend's words; the work order's totals
 // (block items, periphery tiles, quarter tiles, costs), histogram and cursors.
 constexpr int kCtrNext = 0;
