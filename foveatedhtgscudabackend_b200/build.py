@@ -41,7 +41,7 @@ UNITS = [
     ("fhtgs_group.cu", []),
 ]
 HEADERS = ["fhtgs_types.cuh", "fhtgs_math.cuh", "fhtgs_kernels.cuh", "fhtgs_internal.h", "fhtgs_route.h",
-           "fhtgs_order.h"]
+           "fhtgs_order.h", "fhtgs_cull.cuh"]
 
 
 def nvcc() -> str:
