@@ -2251,11 +2251,14 @@ __device__ __forceinline__ void blend_split_records(const FrameParams& fp, const
     __threadfence();
     const char* base = sp.scratch + seg0 * stride;
     const int R = sp.recs;
-    uint32_t most = 0;
+    const TilePixels pp = tile_pixels<RW, 0, 2>(fp, fb, packed, 0);
+    const ViewParams& vp = fb.views[pp.v];
+    uint32_t most = 0;  // of the samples inside the image; the others' records resolve to nothing
     for (uint32_t k = 1; k < S; ++k)
 #pragma unroll
         for (int i = 0; i < 2; ++i)
-            most = max(most, __ldcg(reinterpret_cast<const uint32_t*>(base + k * stride) + tid + i * kBlendThreads));
+            if (pp.x < vp.width && pp.y[i] < vp.height)
+                most = max(most, __ldcg(reinterpret_cast<const uint32_t*>(base + k * stride) + tid + i * kBlendThreads));
     const uint32_t warp_most = __reduce_max_sync(0xffffffffu, most);
     if ((tid & 31) == 0 && warp_most > 0) atomicMax(&fb.counters[kCtrSplitRecMax], warp_most);
     if (__syncthreads_or(most > static_cast<uint32_t>(R))) {
@@ -2263,8 +2266,6 @@ __device__ __forceinline__ void blend_split_records(const FrameParams& fp, const
         blend_tile<K, RW, 0, 2, 1>(fp, fb, packed, 0, true, sm, SegWalk{0u, 1u, 0, 0, nullptr});
         return;
     }
-    const TilePixels pp = tile_pixels<RW, 0, 2>(fp, fb, packed, 0);
-    const ViewParams& vp = fb.views[pp.v];
     for (int px = 0; px < 2; ++px) {
         const int py_i = px == 0 ? pp.y[0] : pp.y[1], at = tid + px * kBlendThreads;
         if (pp.x >= vp.width || py_i >= vp.height) continue;
