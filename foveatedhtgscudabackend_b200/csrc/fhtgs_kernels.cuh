@@ -2186,45 +2186,59 @@ __device__ __forceinline__ void split_replay(const FrameParams& fp, const FrameB
     const TilePixels pp = tile_pixels<RW, 0, 2>(fp, fb, packed, 0);
     const ViewParams& vp = fb.views[pp.v];
     constexpr uint32_t kChunk = 4;  // steps whose log entries are loaded before any is replayed
+    // both pixels of the thread side by side: the replay of one pixel is a serial chain behind its
+    // loads, two fill each other's waits
+    float tail_T[2];
+    float4 tail[2];
+    Frag core[2][K];
+    bool inside[2];
+#pragma unroll
     for (int px = 0; px < 2; ++px) {
-        const int py_i = px == 0 ? pp.y[0] : pp.y[1];
-        if (pp.x >= vp.width || py_i >= vp.height) continue;
-        float tail_T = 1.0f;
-        float4 tail = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        Frag core[K];
+        inside[px] = pp.x < vp.width && pp.y[px] < vp.height;
+        tail_T[px] = 1.0f;
+        tail[px] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
-        for (int k = 0; k < K; ++k) { core[k].depth = 3.402823466e+38f; core[k].color = 0u; }
-        for (uint32_t k = 0; k < S; ++k) {
-            const char* b = sp.pool + 256ull * sp.seg_unit[seg0 + k];
-            const uint32_t n = __ldcg(reinterpret_cast<const uint32_t*>(b) + group);
-            const float4* col = reinterpret_cast<const float4*>(b + 256u * split_log_pos_unit()) +
-                                static_cast<size_t>(group) * log_stride;
-            const float2* fr = reinterpret_cast<const float2*>(b + 256u * split_log_frag_unit(log_stride)) +
-                               static_cast<size_t>(group) * log_stride * 16u + (lane & 7) + 8 * px;
-            for (uint32_t t0 = 0; t0 < n; t0 += kChunk) {
-                float2 ads[kChunk];
-                float4 cs[kChunk];
+        for (int k = 0; k < K; ++k) { core[px][k].depth = 3.402823466e+38f; core[px][k].color = 0u; }
+    }
+    for (uint32_t k = 0; k < S; ++k) {
+        const char* b = sp.pool + 256ull * sp.seg_unit[seg0 + k];
+        const uint32_t n = __ldcg(reinterpret_cast<const uint32_t*>(b) + group);
+        const float4* col = reinterpret_cast<const float4*>(b + 256u * split_log_pos_unit()) +
+                            static_cast<size_t>(group) * log_stride;
+        const float2* fr = reinterpret_cast<const float2*>(b + 256u * split_log_frag_unit(log_stride)) +
+                           static_cast<size_t>(group) * log_stride * 16u + (lane & 7);
+        for (uint32_t t0 = 0; t0 < n; t0 += kChunk) {
+            float2 ads[kChunk][2];
+            float4 cs[kChunk];
 #pragma unroll
-                for (uint32_t i = 0; i < kChunk; ++i) {
-                    const bool ok = t0 + i < n;
-                    ads[i] = ok ? __ldcg(fr + (t0 + i) * 16u) : make_float2(-1.0f, 0.0f);
-                    cs[i] = ok ? __ldcg(col + t0 + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                }
+            for (uint32_t i = 0; i < kChunk; ++i) {
+                const bool ok = t0 + i < n;
 #pragma unroll
-                for (uint32_t i = 0; i < kChunk; ++i) {
-                    const float alpha = ads[i].x;
+                for (int px = 0; px < 2; ++px)
+                    ads[i][px] = ok && inside[px] ? __ldcg(fr + (t0 + i) * 16u + 8 * px) : make_float2(-1.0f, 0.0f);
+                cs[i] = ok ? __ldcg(col + t0 + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
+#pragma unroll
+            for (uint32_t i = 0; i < kChunk; ++i) {
+#pragma unroll
+                for (int px = 0; px < 2; ++px) {
+                    const float alpha = ads[i][px].x;
                     if (alpha < 0.0f) continue;  // not a fragment
                     float4 pm = make_float4(cs[i].x * alpha, cs[i].y * alpha, cs[i].z * alpha, alpha);
-                    if (alpha >= kMinAlphaCore && ads[i].y < core[K - 1].depth) pm = unpack_rgba(core_insert<K>(core, ads[i].y, pm));
+                    if (alpha >= kMinAlphaCore && ads[i][px].y < core[px][K - 1].depth)
+                        pm = unpack_rgba(core_insert<K>(core[px], ads[i][px].y, pm));
                     const float pt = 1.0f - pm.w;
-                    tail += pm;
-                    tail_T *= pt;
+                    tail[px] += pm;
+                    tail_T[px] *= pt;
                 }
             }
         }
-        blend_resolve<K>(fp, vp, core, tail, tail_T, __uint2float_rn(static_cast<uint32_t>(pp.x)),
-                         __uint2float_rn(static_cast<uint32_t>(py_i)), pp.is_fovea ? vp.image : vp.work, pp.x, py_i);
     }
+#pragma unroll
+    for (int px = 0; px < 2; ++px)
+        if (inside[px])
+            blend_resolve<K>(fp, vp, core[px], tail[px], tail_T[px], __uint2float_rn(static_cast<uint32_t>(pp.x)),
+                             __uint2float_rn(static_cast<uint32_t>(pp.y[px])), pp.is_fovea ? vp.image : vp.work, pp.x, pp.y[px]);
 }
 
 // The records mode's segment and merge.  The last of the tile's segments to finish merges them:
@@ -2266,38 +2280,67 @@ __device__ __forceinline__ void blend_split_records(const FrameParams& fp, const
         blend_tile<K, RW, 0, 2, 1>(fp, fb, packed, 0, true, sm, SegWalk{0u, 1u, 0, 0, nullptr});
         return;
     }
+    // both pixels of the thread side by side, see split_replay
+    Frag core[2][K];
+    float4 tail[2];
+    float tail_T[2];
+    bool inside[2];
+#pragma unroll
     for (int px = 0; px < 2; ++px) {
-        const int py_i = px == 0 ? pp.y[0] : pp.y[1], at = tid + px * kBlendThreads;
-        if (pp.x >= vp.width || py_i >= vp.height) continue;
-        Frag core[K];
+        const int at = tid + px * kBlendThreads;
+        inside[px] = pp.x < vp.width && pp.y[px] < vp.height;
         const float* cd = reinterpret_cast<const float*>(base);
         const uint32_t* cc = reinterpret_cast<const uint32_t*>(base + K * 4 * NT);
 #pragma unroll
         for (int k = 0; k < K; ++k) {
-            core[k].depth = __ldcg(cd + k * NT + at);
-            core[k].color = __ldcg(cc + k * NT + at);
+            core[px][k].depth = __ldcg(cd + k * NT + at);
+            core[px][k].color = __ldcg(cc + k * NT + at);
         }
-        float4 tail = __ldcg(reinterpret_cast<const float4*>(base + 2 * K * 4 * NT) + at);
-        float tail_T = __ldcg(reinterpret_cast<const float*>(base + (2 * K + 4) * 4 * NT) + at);
-        for (uint32_t k = 1; k < S; ++k) {
-            const char* b = base + k * stride;
-            const uint32_t n = __ldcg(reinterpret_cast<const uint32_t*>(b) + at);
-            tail += __ldcg(reinterpret_cast<const float4*>(b + 4 * NT) + at);
-            tail_T *= __ldcg(reinterpret_cast<const float*>(b + 5 * 4 * NT) + at);
-            const float* rd = reinterpret_cast<const float*>(b + 6 * 4 * NT);
-            const float4* rp = reinterpret_cast<const float4*>(b + (6 + R) * 4 * NT);
-#pragma unroll 4
-            for (uint32_t r = 0; r < n; ++r) {
-                const float depth = __ldcg(rd + r * NT + at);
-                float4 pm = __ldcg(rp + r * NT + at);
-                if (depth < core[K - 1].depth) pm = unpack_rgba(core_insert<K>(core, depth, pm));
-                tail += pm;
-                tail_T *= 1.0f - pm.w;
-            }
-        }
-        blend_resolve<K>(fp, vp, core, tail, tail_T, __uint2float_rn(static_cast<uint32_t>(pp.x)),
-                         __uint2float_rn(static_cast<uint32_t>(py_i)), pp.is_fovea ? vp.image : vp.work, pp.x, py_i);
+        tail[px] = __ldcg(reinterpret_cast<const float4*>(base + 2 * K * 4 * NT) + at);
+        tail_T[px] = __ldcg(reinterpret_cast<const float*>(base + (2 * K + 4) * 4 * NT) + at);
     }
+    for (uint32_t k = 1; k < S; ++k) {
+        const char* b = base + k * stride;
+        const float* rd = reinterpret_cast<const float*>(b + 6 * 4 * NT) + tid;
+        const float4* rp = reinterpret_cast<const float4*>(b + (6 + R) * 4 * NT) + tid;
+        uint32_t n[2];
+#pragma unroll
+        for (int px = 0; px < 2; ++px) {
+            const int at = tid + px * kBlendThreads;
+            n[px] = inside[px] ? __ldcg(reinterpret_cast<const uint32_t*>(b) + at) : 0u;
+            tail[px] += __ldcg(reinterpret_cast<const float4*>(b + 4 * NT) + at);
+            tail_T[px] *= __ldcg(reinterpret_cast<const float*>(b + 5 * 4 * NT) + at);
+        }
+        const uint32_t n_max = max(n[0], n[1]);
+        constexpr uint32_t kChunk = 4;  // records loaded before any is replayed
+        for (uint32_t r0 = 0; r0 < n_max; r0 += kChunk) {
+            float depth[kChunk][2];
+            float4 pms[kChunk][2];
+#pragma unroll
+            for (uint32_t i = 0; i < kChunk; ++i)
+#pragma unroll
+                for (int px = 0; px < 2; ++px) {
+                    const uint32_t at = (r0 + i) * NT + px * kBlendThreads;
+                    const bool ok = r0 + i < n[px];  // else FLT_MAX: not inserted, adds nothing
+                    depth[i][px] = ok ? __ldcg(rd + at) : 3.402823466e+38f;
+                    pms[i][px] = ok ? __ldcg(rp + at) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                }
+#pragma unroll
+            for (uint32_t i = 0; i < kChunk; ++i)
+#pragma unroll
+                for (int px = 0; px < 2; ++px) {
+                    float4 pm = pms[i][px];
+                    if (depth[i][px] < core[px][K - 1].depth) pm = unpack_rgba(core_insert<K>(core[px], depth[i][px], pm));
+                    tail[px] += pm;
+                    tail_T[px] *= 1.0f - pm.w;
+                }
+        }
+    }
+#pragma unroll
+    for (int px = 0; px < 2; ++px)
+        if (inside[px])
+            blend_resolve<K>(fp, vp, core[px], tail[px], tail_T[px], __uint2float_rn(static_cast<uint32_t>(pp.x)),
+                             __uint2float_rn(static_cast<uint32_t>(pp.y[px])), pp.is_fovea ? vp.image : vp.work, pp.x, pp.y[px]);
 }
 
 // One segment of a split full-resolution tile (split list entry g): the exact split's log and
