@@ -100,7 +100,8 @@ constexpr float kCoreCutoff = 5.0910620f;
 // two samples a lane (PX 2), or two groups, one per 16 lanes (PX 1, half items).  CLS 0: a
 // full-resolution tile (16 x 16 samples, 16 groups: the whole block, or half of them for a half
 // item); CLS 1: a periphery tile (8 x 8 samples at stride 2, four groups, one warp); CLS 2: a
-// ring-mode quarter tile (4 x 4 samples at stride 4, one group: a warp blends four tiles).
+// ring-mode quarter tile (4 x 4 samples at stride 4, one group: a warp blends four tiles, or with
+// PX 1 one whose list is long).
 // RW (fhtgs_tuning.blend_warp_width) gives the group rectangle: 8: 4 x 4, 16: 8 x 2, 4: 2 x 8.
 template <int RW, int CLS>
 struct GroupShape {

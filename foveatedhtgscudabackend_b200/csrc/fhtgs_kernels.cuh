@@ -1328,15 +1328,6 @@ int launch_ranges(const FrameParams& fp, const FrameBuffers& fb, int n_sms, cuda
 // work ordering for the persistent blend (bucketed longest-processing-time first).
 // The items, their words and their places: fhtgs_order.h.
 // ------------------------------------------------------------------------------------------
-// Estimated duration of an item in list entries of a full item: per entry of its (longest) list,
-// plus the item's fixed cost.  Measured at five blocks per SM: 168 ns per entry of a full item and
-// 90 of a half item (stereo frame), 144 and 208 of a full and a periphery item (6M Gaussians,
-// rings), about 5 us fixed.
-constexpr float kCostHalf = 0.6f, kCostLow = 1.6f, kCostQuarter = 2.5f, kCostItem = 32.0f;
-// A full-resolution tile becomes two half items when its list is longer than this share of the
-// frame's instances per SM: its walk would then outlast the frame at five blocks per SM.
-constexpr float kHalfShare = 0.16f;
-
 // Resident blocks per SM.  More blocks hide more latency (relative throughput of 1 to 5 blocks,
 // measured on a 12-view frame: 1, 1.75, 2.29, 2.64, 2.86), but each block then walks slower, and
 // a frame ends with its longest item.  With u = longest item / (all items per SM), the time at b
@@ -1391,14 +1382,21 @@ __device__ __forceinline__ uint16_t* order_decisions(const FrameParams& fp, cons
     return reinterpret_cast<uint16_t*>(fb.work_order[1] + 2 * static_cast<size_t>(fp.n_views) * fp.max_large);
 }
 
-// Estimated duration of a tile's item (class 2: full or half), see kCostHalf.
-__device__ __forceinline__ float item_cost(int cls, uint32_t len, bool halves) {
-    const float c = cls == 2 ? 1.0f : cls == 1 ? kCostLow : kCostQuarter;
-    return c * (halves ? kCostHalf : 1.0f) * static_cast<float>(len) + kCostItem;
+// Estimated duration of a tile's item (class 2, 1: whole or half; 0: among sixteen or alone on a
+// warp), see kCostHalf.
+__device__ __forceinline__ float item_cost(int cls, uint32_t len, bool apart) {
+    const float c = cls == 2 ? (apart ? kCostHalf : 1.0f)
+                  : cls == 1 ? (apart ? kCostLow * kCostHalf : kCostLow)
+                             : (apart ? kCostAlone : kCostQuarter);
+    return c * static_cast<float>(len) + kCostItem;
 }
-// Does the tile become two half items (half_threshold)?
-__device__ __forceinline__ bool blend_halves(int cls, uint32_t len, uint32_t half_len) {
-    return cls == 2 ? len > half_len : cls == 1 && kCostLow * static_cast<float>(len) > static_cast<float>(half_len);
+// Is the tile taken apart (half_threshold): into two half items, a quarter tile alone on a warp?  (A
+// quarter tile among sixteen is staged by 8 lanes, 24 Gaussians at a time, and takes 330-530 ns per
+// list entry; alone on a warp about 120.  16 mixed views, whose longest quarter list has 33,383
+// entries: blend 10.4 -> 4.5 ms.)
+__device__ __forceinline__ bool blend_apart(int cls, uint32_t len, uint32_t half_len) {
+    const float c = cls == 2 ? 1.0f : cls == 1 ? kCostLow : kCostQuarter;
+    return cls == 2 ? len > half_len : c * static_cast<float>(len) > static_cast<float>(half_len);
 }
 
 // List length above which a full-resolution tile is blended as two half items.
@@ -1495,11 +1493,12 @@ __global__ void __launch_bounds__(256) order_hist_kernel(FrameParams fp, FrameBu
                 continue;
             }
         }
-        const bool halves = blend_halves(cls, len, half_len);
-        const float cost = item_cost(cls, len, halves);
+        const bool apart = blend_apart(cls, len, half_len), halves = apart && cls != 0, alone = apart && cls == 0;
+        const float cost = item_cost(cls, len, apart);
+        const int list = alone ? 1 : cls;  // a quarter tile alone is an entry of a low item
         longest = fmaxf(longest, cost);
-        cost_sum += cost * (halves ? 2.0f : 1.0f) / static_cast<float>(cls == 2 ? 1u : cls == 1 ? kLowTiles : kQuarterTiles);
-        const uint16_t word = order_word(cls * kCostBuckets + cost_bucket(cost), halves);
+        cost_sum += cost * (halves ? 2.0f : 1.0f) / static_cast<float>(list == 2 ? 1u : list == 1 ? kLowTiles : kQuarterTiles);
+        const uint16_t word = order_word(list * kCostBuckets + cost_bucket(cost), halves, alone);
         order_decisions(fp, fb)[static_cast<size_t>(v) * fp.max_large + j] = word;
         atomicAdd(&hist[order_bucket(word)], order_entries(word));
     }
@@ -1869,7 +1868,8 @@ __device__ __forceinline__ TilePixels tile_pixels(const FrameParams& fp, const F
 }
 
 // Blends one tile, or half of one (PX 1: `half`), with a team of threads: the block (CLS 0), a
-// warp (CLS 1) or 8 lanes (CLS 2; `live` false: no tile for this group).  The team stages its tile's list
+// warp (CLS 1; CLS 2 with PX 1: a quarter tile alone, its one group on the lower 16 lanes) or 8
+// lanes (CLS 2 with PX 2; `live` false: no tile for this group).  The team stages its tile's list
 // kBlendPerThread Gaussians a thread at a time; every thread culls its own against the tile's sample groups, each
 // group's survivors become its list, and the warp walks its groups' lists side by side, in list
 // order.  Which pairs are culled (pairs that cannot pass the alpha test) never changes a
@@ -1878,16 +1878,17 @@ template <int K, int RW, int CLS, int PX, int SEG = 0>
 __device__ __forceinline__ void blend_tile(const FrameParams& fp, const FrameBuffers& fb, uint32_t packed, int half, bool live,
                                            BlendSmem& sm, const SegWalk sw = SegWalk{0u, 1u, 0, 0, nullptr}) {
     using G = GroupShape<RW, CLS>;
-    constexpr uint32_t TEAM = CLS == 0 ? kBlendThreads : CLS == 1 ? 32 : 8;
+    constexpr bool WARP = CLS == 1 || (CLS == 2 && PX == 1);  // a warp is the team
+    constexpr uint32_t TEAM = CLS == 0 ? kBlendThreads : WARP ? 32 : 8;
     constexpr uint32_t BATCH = kBlendPerThread * TEAM;
     constexpr bool log_mode = SEG == 3;  // the exact split's segment: log the fragments only
     constexpr int NT = kSplitPx;
     constexpr int LPG = 16 / PX, GPW = 32 / LPG;  // lanes per group, groups per warp
     constexpr uint32_t EPS = 2 / PX;              // list entries a step evaluates
-    static_assert(PX == 2 || (CLS != 2 && SEG == 0), "no halves of quarter tiles and of split segments");
+    static_assert(PX == 2 || SEG == 0, "no halves of split segments");
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, grp = lane / LPG;
-    const uint32_t team_tid = CLS == 0 ? tid : CLS == 1 ? lane : lane & 7;
-    const uint32_t team_base = CLS == 0 ? 0u : CLS == 1 ? warp * BATCH : (warp * 4 + grp) * BATCH;
+    const uint32_t team_tid = CLS == 0 ? tid : WARP ? lane : lane & 7;
+    const uint32_t team_base = CLS == 0 ? 0u : WARP ? warp * BATCH : (warp * 4 + grp) * BATCH;
     const uint32_t lanemask_lt = (1u << lane) - 1u;
     const TilePixels pp = tile_pixels<RW, CLS, PX>(fp, fb, packed, half);
     const ViewParams& vp = fb.views[pp.v];
@@ -1928,7 +1929,7 @@ __device__ __forceinline__ void blend_tile(const FrameParams& fp, const FrameBuf
         for (int k = 0; k < K; ++k) { core[i][k].depth = 3.402823466e+38f; core[i][k].color = 0u; }
     }
 
-    for (uint32_t start = range.x; CLS == 2 ? __any_sync(0xffffffffu, start < range.y) : start < range.y; start += BATCH) {
+    for (uint32_t start = range.x; CLS == 2 && !WARP ? __any_sync(0xffffffffu, start < range.y) : start < range.y; start += BATCH) {
         const uint32_t n_batch = start < range.y ? min(BATCH, range.y - start) : 0u;
         if (CLS == 0) __syncthreads(); else __syncwarp();
         uint32_t mask[kBlendPerThread];
@@ -1947,13 +1948,13 @@ __device__ __forceinline__ void blend_tile(const FrameParams& fp, const FrameBuf
                 mask[h] = reached_groups<RW, CLS, ROWS_USED>(P1, P2, P4, c.w, static_cast<float>(pp.ox),
                                                              static_cast<float>(pp.oy), row0, valid, sm.zmin[slot]);
             }
-            if (CLS != 2) sm.mask[slot] = static_cast<uint16_t>(mask[h]);
+            if (CLS == 0 || WARP) sm.mask[slot] = static_cast<uint16_t>(mask[h]);
         }
         if (CLS == 0) __syncthreads(); else __syncwarp();
         // the lists of this warp's groups: the staged slots whose mask has the group's bit
         uint32_t n_mine, n_max;
         uint32_t step0 = 0;
-        if constexpr (CLS != 2) {
+        if constexpr (CLS == 0 || WARP) {
             uint32_t n[GPW] = {};
             for (uint32_t c0 = 0; c0 < n_batch; c0 += 32) {
                 const uint32_t slot = team_base + c0 + lane;
@@ -2170,7 +2171,7 @@ __device__ __forceinline__ void blend_tile(const FrameParams& fp, const FrameBuf
     } else {
 #pragma unroll
         for (int i = 0; i < PX; ++i)
-            if (live && pp.x < vp.width && pp.y[i] < vp.height)
+            if (live && (CLS != 2 || PX == 2 || grp == 0) && pp.x < vp.width && pp.y[i] < vp.height)
                 blend_resolve<K>(fp, vp, core[i], tail[i], tail_T[i], pixel_x, pixel_y[i], pp.is_fovea ? vp.image : vp.work,
                                  pp.x, pp.y[i]);
     }
@@ -2427,6 +2428,7 @@ __global__ void __launch_bounds__(kBlendThreads, blend_blocks(K)) blend_kernel(F
             if (i < n_low) {
                 const uint32_t tile = runs[i], part = tile >> kItemKindShift;
                 if (part == kItemFull) blend_tile<K, RW, 1, 2>(fp, fb, tile, 0, true, sm);
+                else if (part == kItemQuarter) blend_tile<K, RW, 2, 1>(fp, fb, tile, 0, true, sm);
                 else blend_tile<K, RW, 1, 1>(fp, fb, tile, static_cast<int>(part - kItemHalf), true, sm);
             }
         } else {

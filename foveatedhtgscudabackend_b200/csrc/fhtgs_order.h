@@ -7,11 +7,13 @@
 //   full    a full-resolution tile, two pixels a thread
 //   half    the upper or lower half of a full-resolution tile, one pixel a thread: the tiles
 //           whose walk alone would outlast the frame's mean work per block
-//   low     four periphery tiles, or halves of them, one per warp
-//   quarter sixteen ring-mode quarter tiles, four per warp
+//   low     four periphery tiles, halves of them, or ring-mode quarter tiles with long lists, one
+//           per warp
+//   quarter sixteen other quarter tiles, four per warp
 // An item word is kind << 29 | view << 21 | index into the view's work_full list, or kind << 29 |
 // item number for the last two, whose tiles lie in a second list, the runs (the same word, with
-// the index into work_low), longest first: the periphery tiles of all views, then the quarter tiles.
+// the index into work_low; kind kItemQuarter: a quarter tile that a warp blends alone), longest first:
+// the entries of all views' low items, then those of the quarter items.
 #pragma once
 #include <stdint.h>
 
@@ -24,7 +26,7 @@
 namespace fhtgs {
 
 constexpr int kCostBuckets = 130;                // per tile class: estimated duration in quarter octaves
-constexpr int kOrderBuckets = 3 * kCostBuckets;  // quarter (class 0), periphery (1), full-resolution (2)
+constexpr int kOrderBuckets = 3 * kCostBuckets;  // quarter (class 0), low (1), full-resolution (2)
 
 constexpr uint32_t kItemFull = 0u, kItemHalf = 1u /* and 2 */, kItemLow = 3u, kItemQuarter = 4u;
 constexpr int kItemKindShift = 29, kItemViewShift = 21;
@@ -35,14 +37,29 @@ FHTGS_HD uint32_t item_index(uint32_t packed) { return packed & kItemIndexMask; 
 // Tiles (or halves) of a low / quarter item.
 constexpr uint32_t kLowTiles = 4, kQuarterTiles = 16;
 
+// Estimated duration of an item in list entries of a full item: per entry of its (longest) list,
+// plus the item's fixed cost (about 5 us).  Measured per entry at 1 / 5 blocks per SM (K = 8): a full
+// item 69-88 / 167-170 ns, a half item 30-49 / 47-91, a low item of whole tiles 137-196 / 303-339, of
+// halves 72-95 / 134-136 (4 blocks), a quarter item 331-382 / 462-534, of quarter tiles alone 117-120 /
+// 151 (3 blocks).  The factors are those ratios where the frames are fastest: half 0.6 (0.5: 6M with
+// rings 14.26 -> 16.09 ms of blend, the stereo frame with rings 2.60 -> 2.77), low 1.6 (1.4: 14.82 and
+// 2.62; 2.0: 15.62 and 2.77), quarter 4 (2.5: 64 mixed views with rings 9.47 instead of 7.45 ms), alone
+// 1.2 (1.6: 16 mixed views 5.61 instead of 4.47 ms).
+constexpr float kCostHalf = 0.6f, kCostLow = 1.6f, kCostQuarter = 4.0f, kCostAlone = 1.2f, kCostItem = 32.0f;
+// A full-resolution tile becomes two half items when its list is longer than this share of the
+// frame's instances per SM: its walk would then outlast the frame at five blocks per SM.
+constexpr float kHalfShare = 0.16f;
+
 // What the order decides about a tile: its bucket (class above duration bucket), and whether it
-// becomes two half items.  Decided once, when the buckets are counted, and kept: the buckets'
-// runs hold exactly the counted entries, whatever the estimate's rounding.
+// becomes two half items or, a quarter tile, an entry of a low item.  Decided once, when the buckets
+// are counted, and kept: the buckets' runs hold exactly the counted entries, whatever the
+// estimate's rounding.
 constexpr uint16_t kOrderSplit = 0xffffu;  // a tile of the split blend: no entry
-FHTGS_HD uint16_t order_word(int bucket, bool halves) {
-    return static_cast<uint16_t>(bucket | (halves ? 0x8000 : 0));
+FHTGS_HD uint16_t order_word(int bucket, bool halves, bool alone) {
+    return static_cast<uint16_t>(bucket | (halves ? 0x8000 : 0) | (alone ? 0x4000 : 0));
 }
-FHTGS_HD int order_bucket(uint16_t word) { return word & 0x7fff; }
+FHTGS_HD int order_bucket(uint16_t word) { return word & 0x3fff; }
+FHTGS_HD bool order_alone(uint16_t word) { return (word & 0x4000) != 0; }
 FHTGS_HD uint32_t order_entries(uint16_t word) { return (word & 0x8000) ? 2u : 1u; }
 
 // The frame's totals.  `base[b]`: entries in buckets above b (all classes, descending).
@@ -74,7 +91,7 @@ struct OrderTotals {
     FHTGS_HD void put(uint16_t word, uint32_t at, uint32_t packed, uint32_t* out, uint32_t* runs) const {
         const int b = order_bucket(word), cls = b / kCostBuckets, d = b - cls * kCostBuckets;
         const bool halves = order_entries(word) == 2u;
-        const uint32_t kind = halves ? kItemHalf : kItemFull;
+        const uint32_t kind = halves ? kItemHalf : order_alone(word) ? kItemQuarter : kItemFull;
         uint32_t* list = cls == 2 ? out + low_items(d + 1) + quarter_items(d + 1) + at : runs + (at - full);
         list[0] = (kind << kItemKindShift) | packed;
         if (halves) list[1] = ((kind + 1u) << kItemKindShift) | packed;

@@ -67,7 +67,8 @@ def test_every_tile_once_longest_first(order, counts, spread, split):
     n = len(cls)
     bucket = rng.integers(BUCKETS - spread, BUCKETS, n) if spread < BUCKETS else rng.integers(0, BUCKETS, n)
     halves = (rng.random(n) < 0.4) & (cls > 0)
-    word = (cls * BUCKETS + bucket + (halves << 15)).astype(np.uint16)
+    alone = (rng.random(n) < 0.3) & (cls == 0)  # quarter tiles that a warp blends alone: entries of low items
+    word = (np.where(alone, 1, cls) * BUCKETS + bucket + (halves << 15) + (alone << 14)).astype(np.uint16)
     gone = split & (cls == 2) & (rng.random(n) < 0.3)
     word[gone] = 0xFFFF
     index = np.concatenate([np.arange(counts[0]), np.arange(counts[1] + counts[2])]).astype(np.uint32)
@@ -100,7 +101,7 @@ def test_every_tile_once_longest_first(order, counts, spread, split):
         assert b <= last, "a longer bucket after a shorter one"
         last = b
     assert numbers[3] == list(range(-(-n_low // 4))) and numbers[4] == list(range(-(-n_quarter // 16)))
-    want = [(i, k) for i in range(n) if not gone[i] for k in ((1, 2) if halves[i] else (0,))]
+    want = [(i, k) for i in range(n) if not gone[i] for k in ((1, 2) if halves[i] else (4,) if alone[i] else (0,))]
     assert sorted(seen) == want
 
 
@@ -108,5 +109,5 @@ def test_scatter_takes_the_counted_decision():
     src = open(os.path.join(CSRC, "fhtgs_kernels.cuh")).read()
     body = re.search(r"order_scatter_kernel\(FrameParams.*?\n}\n", src, re.S).group(0)
     assert "order_decisions(" in body
-    for estimate in ("item_cost(", "blend_halves(", "cost_bucket(", "half_threshold("):
+    for estimate in ("item_cost(", "blend_halves(", "blend_apart(", "cost_bucket(", "half_threshold("):
         assert estimate not in body, f"the scatter kernel makes its own {estimate}...)"
