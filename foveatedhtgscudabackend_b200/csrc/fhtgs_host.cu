@@ -513,7 +513,7 @@ fhtgs_status render_impl(fhtgs_context ctx, const fhtgs_primitives* prims, const
     mark(2);
     if (nbp > 0) {
         n += ks.scan_blocks(fp, fb, stream);
-        n += ks.create_instances(fp, fb, stream);
+        n += ks.create_instances(fp, fb, ctx->n_sms, stream);
     }
     mark(3);
     n += ks.sort(fp, fb, stream);

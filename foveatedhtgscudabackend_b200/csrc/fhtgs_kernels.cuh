@@ -783,11 +783,11 @@ __device__ __forceinline__ void count_key(uint32_t* s_hist, int passes, uint32_t
     for (int p = 0; p < passes; ++p) atomicAdd(&s_hist[p * kSortBins + ((key >> (p * kSortRadixBits)) & (kSortBins - 1))], 1u);
 }
 
-// Blocks of the creation over all views; each loops over chunks of 256 Gaussians, so that the
+// Blocks of the creation per SM, over all views; each loops over chunks of 256 Gaussians, so that the
 // digit counts of a frame of many views reach the few global counters once per block instead of
 // once per chunk (12 views of 1M: scan + create 0.483 -> 0.295 ms; stereo 1M 0.129 -> 0.125 ms;
 // a quarter as many blocks leave the uneven chunks unbalanced: 0.157 ms stereo).
-constexpr int kCreateBlocks = 32 * 148;
+constexpr int kCreateBlocksPerSm = 32;
 
 template <typename KeyT>
 __global__ void __launch_bounds__(kPrimBlock) create_instances_kernel(FrameParams fp, FrameBuffers fb) {
@@ -908,9 +908,9 @@ __global__ void __launch_bounds__(kPrimBlock) create_instances_kernel(FrameParam
     }
 }
 
-int launch_create(const FrameParams& fp, const FrameBuffers& fb, cudaStream_t s) {
+int launch_create(const FrameParams& fp, const FrameBuffers& fb, int n_sms, cudaStream_t s) {
     if (fp.n_blocks_prim == 0) return 0;
-    const int per_view = (kCreateBlocks + fp.n_views - 1) / fp.n_views;
+    const int per_view = (kCreateBlocksPerSm * n_sms + fp.n_views - 1) / fp.n_views;
     dim3 grid(fp.n_blocks_prim < per_view ? fp.n_blocks_prim : per_view, fp.n_views);
     if (fp.key_u32) create_instances_kernel<uint32_t><<<grid, kPrimBlock, 0, s>>>(fp, fb);
     else create_instances_kernel<uint16_t><<<grid, kPrimBlock, 0, s>>>(fp, fb);

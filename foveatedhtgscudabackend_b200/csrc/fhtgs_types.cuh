@@ -232,7 +232,7 @@ struct KernelSet {
     int (*classify)(const FrameParams& fp, const FrameBuffers& fb, cudaStream_t s);
     int (*preprocess)(const FrameParams& fp, const FrameBuffers& fb, const Gaussians& g, cudaStream_t s);
     int (*scan_blocks)(const FrameParams& fp, const FrameBuffers& fb, cudaStream_t s);
-    int (*create_instances)(const FrameParams& fp, const FrameBuffers& fb, cudaStream_t s);
+    int (*create_instances)(const FrameParams& fp, const FrameBuffers& fb, int n_sms, cudaStream_t s);
     int (*sort)(const FrameParams& fp, FrameBuffers& fb, cudaStream_t s);
     int (*ranges)(const FrameParams& fp, const FrameBuffers& fb, int n_sms, cudaStream_t s);
     int (*order)(const FrameParams& fp, const FrameBuffers& fb, const SplitArgs& sp, int n_sms, cudaStream_t s);
