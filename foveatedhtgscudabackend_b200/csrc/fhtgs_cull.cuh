@@ -23,14 +23,10 @@ __device__ __forceinline__ float sqrt_approx(float x) {
 }
 #endif
 
-// Pixel-space bounding box of a Gaussian's cutoff ellipse, evaluated about the projected
-// mean (x0 = P1.w / P4.w) so that no large terms cancel.  Returns false when the box is
+// Pixel-space bounding box of a Gaussian's cutoff ellipse (rc = 2 ln(255 opacity)), evaluated about
+// the projected mean (x0 = P1.w / P4.w) so that no large terms cancel.  Returns false when the box is
 // unbounded (camera inside the cutoff quadric or mean behind it): no culling then.
-__device__ __forceinline__ bool cutoff_box(const float4 P1, const float4 P2, const float4 P4, float opacity,
-                                           float4& box, bool& never) {
-    never = false;
-    const float rc = 2.0f * __logf(opacity * kMinAlphaRcp);
-    if (rc < 0.0f) { never = true; return true; }  // alpha <= opacity < 1/255 everywhere
+__device__ __forceinline__ bool cutoff_box(const float4 P1, const float4 P2, const float4 P4, float rc, float4& box) {
     if (!(P4.w > 0.0f) || !(rc > 0.0f)) return false;
     const float3 n4 = xyz(P4);
     const float a = P4.w * P4.w - rc * dot(n4, n4);
@@ -115,7 +111,8 @@ struct GroupShape {
 // among `valid`.  The cutoff ellipse about its centre is x = slope y +- hx sqrt(1 - (y / ymax)^2);
 // its x extent over a row of groups gives that row's bits at once (one test per row of groups
 // instead of one per group).  Ellipses that are not clearly ellipses, or out of the range of the
-// approximate arithmetic, are tested by their bounding box; unbounded ones reach every group, and
+// approximate arithmetic (both math flavours use it here: it gates pairs within the margins and
+// reaches no pixel), are tested by their bounding box; unbounded ones reach every group, and
 // so do Gaussians so small (rc |d|^2 at the mean) that the blend's 1 / |d|^2 may overflow:
 // 0 x inf makes their alpha 1 at any pixel of their tiles.
 // Rows row0 .. row0 + ROWS_USED - 1 of groups are tested (a half item's).
@@ -172,9 +169,7 @@ __device__ __forceinline__ uint32_t reached_groups(const float4 P1, const float4
     const float ix = P1.w / P4.w, iy = P2.w / P4.w;
     const float3 c0 = cross(xyz(P1) - ix * n4, xyz(P2) - iy * n4);  // the direction vector d at the mean
     float4 box;
-    bool never;
-    if (!(rc * dot(c0, c0) > 1e-28f) || !cutoff_box(P1, P2, P4, opacity, box, never)) return valid;
-    if (never) return 0u;
+    if (!(rc * dot(c0, c0) > 1e-28f) || !cutoff_box(P1, P2, P4, rc, box)) return valid;
     for (int g = 0; g < G::COLS * G::ROWS; ++g) {
         const float ax0 = ox + static_cast<float>((g % G::COLS) * G::GW) * fS, ax1 = ax0 + static_cast<float>(G::GW - 1) * fS;
         const float ay0 = oy + static_cast<float>((g / G::COLS) * G::GH) * fS, ay1 = ay0 + static_cast<float>(G::GH - 1) * fS;

@@ -1333,7 +1333,11 @@ int launch_ranges(const FrameParams& fp, const FrameBuffers& fb, int n_sms, cuda
 // a frame ends with its longest item.  With u = longest item / (all items per SM), the time at b
 // blocks is about max(1 / throughput(b), u b / throughput(b)): the limits below are where b blocks
 // become better than b + 1.  (Plain view, u = 1.2: blend 0.34 -> 0.20 ms at one block; half-size
-// stereo frame, u = 0.38: 2.43 -> 1.84 ms at three.)
+// stereo frame, u = 0.38: 2.43 -> 1.84 ms at three.)  The limits are those of K = 8; frames at K >= 16,
+// whose registers allow 3 and 2 blocks, agree with them (blend in us at 1 / 2 / 3 blocks, the rule's
+// choice in brackets: K = 16, 300k at 1920x1080 696 / 461 / 558 [2], stereo frame 9342 / 5601 / 4450
+// [3], a clustered 1280x720 view 2360 / 2444 / 2860 [1]; K = 32 912 / 628 [2], 11682 / 7374 [2],
+// 2614 / 2719 [1]).
 __device__ __forceinline__ uint32_t blocks_per_sm(float u, uint32_t most) {
     const uint32_t b = u < 0.21f ? 5u : u < 0.29f ? 4u : u < 0.43f ? 3u : u < 0.87f ? 2u : 1u;
     return b < most ? b : most;
@@ -2498,7 +2502,7 @@ int launch_blend(const FrameParams& fp, const FrameBuffers& fb, const SplitArgs&
 // compose: periphery upsampling / blur and blended cross-fade (restates
 // bilinear_interpolation, bilinear_interpolation_blended, interpolate_and_blur and
 // interpolate_and_blur_blended, interpolation.cuh:11-584), plus clearing of masked tiles.
-// One 256-thread block per large tile; blended tiles use four 64-thread groups.
+// One 64-thread block per non-fovea large tile, four pixels a thread.
 // ------------------------------------------------------------------------------------------
 __device__ __forceinline__ float3 load_rgb(const float* img, int W, int H, int x, int y, bool chw) {
     const int sx = clampi(x, 0, W - 1), sy = clampi(y, 0, H - 1);

@@ -47,7 +47,12 @@ constexpr uint32_t kLowTiles = 4, kQuarterTiles = 16;
 // 1.2 (1.6: 16 mixed views 5.61 instead of 4.47 ms).
 constexpr float kCostHalf = 0.6f, kCostLow = 1.6f, kCostQuarter = 4.0f, kCostAlone = 1.2f, kCostItem = 32.0f;
 // A full-resolution tile becomes two half items when its list is longer than this share of the
-// frame's instances per SM: its walk would then outlast the frame at five blocks per SM.
+// frame's instances per SM: its walk would then outlast the frame at five blocks per SM.  (Blend of
+// the stereo frame in us at 0.06 / 0.1 / 0.13 / 0.16 / 0.2 / 0.26 / never: K = 8 3639 / 3507 / 3369 /
+// 3256 / 3374 / 3450 / 3436, K = 16 4725 / 4633 / 4549 / 4448 / 4318 / 4284 / 4286, K = 32 7509 / 7492 /
+// 7445 / 7374 / 7268 / 7241 / 7240; without halves the plain view takes 287 instead of 190, 300k at
+// 1920x1080 593 instead of 430 at K = 8, 656 / 461 at K = 16, 996 / 625 at K = 32.  At K >= 16, where
+// fewer blocks are resident, a larger share would be 2-4 % better on frames of many tiles.)
 constexpr float kHalfShare = 0.16f;
 
 // What the order decides about a tile: its bucket (class above duration bucket), and whether it

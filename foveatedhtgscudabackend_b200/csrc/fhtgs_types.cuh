@@ -191,7 +191,7 @@ __host__ __device__ constexpr int split_share_blocks(int K) { return K >= 32 ? 2
 // segments on different blocks, merged by the last of them.
 struct SplitArgs {
     float share;           // 0: off
-    int blocks;            // persistent blend blocks of the launch
+    int blocks;            // the block count the share refers to (split_share_blocks per SM)
     int cap;               // segments the scratch holds
     int recs;              // records a later segment keeps per pixel
     int stride;            // bytes of scratch per segment
@@ -200,7 +200,7 @@ struct SplitArgs {
     uint32_t* ctl;         // [cap] per first segment: segments finished
     char* scratch;         // [cap][stride] per-pixel state and records
     // Exact mode (bit-identical images): every segment logs, per pixel and in list order, the
-    // alpha and depth of each Gaussian its warp evaluates; the last segment of a tile replays the
+    // alpha and depth of each Gaussian its group evaluates; the last segment of a tile replays the
     // whole log with the walk's own K-buffer and tail steps.
     int exact;
     uint32_t pool_units;   // 256-byte units of the fragment log
