@@ -118,8 +118,8 @@ def parse(argv=None):
 # clocks during the timed region
 # ------------------------------------------------------------------------------------------
 # DRAM traffic of one blend_kernel<8,8> launch of the headline frame, measured by ncu on B200
-# (353.9 MB read + 45.3 MB written; the kernel gathers ~0.95 GB of records, mostly from L2)
-BLEND_DRAM_BYTES = 399.2e6
+# (320.9 MB read + 40.5 MB written; the kernel gathers ~0.9 GB of records, mostly from L2)
+BLEND_DRAM_BYTES = 361.4e6
 
 
 class ClockSampler:
@@ -545,7 +545,8 @@ def run_ours(a, world, rank, local):
                      "frac": round(achieved / peak_fp32, 4),
                      # DRAM bytes of one blend launch on this workload from one ncu capture
                      # (dram__bytes_read.sum + dram__bytes_write.sum): profiles/blend_kernel_stereo_1M_2x2064x2208.md
-                     "traffic": BLEND_DRAM_BYTES if a.foveation == "reference" and a.n_gaussians == 1_000_000 else None,
+                     "traffic": BLEND_DRAM_BYTES if (a.foveation, a.n_gaussians, a.sh_degree, a.K, a.width, a.height) ==
+                     ("reference", 1_000_000, 3, 8, 2064, 2208) else None,
                      "traffic_unit": "bytes per launch (ncu)",
                      "peak_source": "nominal FP32 SIMT: SMs x 128 lanes x 2 x median SM clock under load",
                      "work": f"{pairs} pixel-Gaussian pairs x {FLOP_PER_PAIR} flop "
