@@ -118,8 +118,8 @@ def parse(argv=None):
 # clocks during the timed region
 # ------------------------------------------------------------------------------------------
 # DRAM traffic of one blend_kernel<8,8> launch of the headline frame, measured by ncu on B200
-# (320.9 MB read + 40.5 MB written; the kernel gathers ~0.9 GB of records, mostly from L2)
-BLEND_DRAM_BYTES = 361.4e6
+# (317.0 MB read + 41.0 MB written; the kernel gathers ~0.9 GB of records, mostly from L2)
+BLEND_DRAM_BYTES = 358.0e6
 
 
 class ClockSampler:

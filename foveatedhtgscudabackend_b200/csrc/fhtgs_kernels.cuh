@@ -1628,9 +1628,9 @@ int launch_order(const FrameParams& fp, const FrameBuffers& fb, const SplitArgs&
 //   - half items (one pixel a lane, two list entries a step: 1.07 times the work of the whole
 //     tile in about half its time) and fewer blocks per SM for frames that end with a few long
 //     tiles (work order).
-// Blend of the stereo frame (1M Gaussians, 2 x 2064x2208, K = 8) 4.87 -> 3.30 ms, of 12 views of
-// 1920x1080 10.65 -> 6.7 ms, of the plain 1280x720 view (100k, K = 4) 0.73 -> 0.18 ms, of a
-// 2 x 1032x1104 frame of the 1M scene 5.3 -> 1.7 ms, of 6M with rings 27.8 -> 16.2 ms, K = 32 at
+// Blend of the stereo frame (1M Gaussians, 2 x 2064x2208, K = 8) 4.87 -> 3.25 ms, of 12 views of
+// 1920x1080 10.65 -> 6.7 ms, of the plain 1280x720 view (100k, K = 4) 0.73 -> 0.17 ms, of a
+// 2 x 1032x1104 frame of the 1M scene 5.9 -> 1.7 ms, of 6M with rings 27.8 -> 15.5 ms, K = 32 at
 // 1280x720 0.72 -> 0.54 ms.
 // ------------------------------------------------------------------------------------------
 struct Frag {
